@@ -12,6 +12,14 @@
 // fixed symmetric operator up to FP32 rounding; the outer FP64 flexible CG
 // absorbs the rest.
 //
+// The gauge (p[0] = 0) is a choice among the solutions of the singular system,
+// not an equation: the outer iteration keeps every row's residual, row 0
+// included, and represents z by x - x[0], so d[0] = p[0] = 0 throughout. With
+// row 0 eliminated (r[0] = z[0] = 0) the cycle saw a residual whose sum was
+// not zero and its output was cut at one cell: 12 flexible-CG iterations to
+// 1e-8 at 128^3 instead of 7 (2.86 ms per carrier step, 1.95 ms now; 256^3
+// 14.3 and 9.8 ms; 64 batched boxes 37.9 and 24.6 ms per step).
+//
 // Launch structure of one cycle: grid-wide kernels for the levels above 32^3
 // cells; one kernel on a thread-block cluster (16 CTAs where the device
 // schedules them) for every level of at most 32^3 cells, the dense coarsest
@@ -87,7 +95,7 @@ public:
     int enqueue_update_first(const GridDev& g, void* state, double* p, double* r0, double* r1, double* d0,
                              double* d1, Partials part, rb200_trace* trace, cudaStream_t s) const;
     // The finish: last red half-sweep of level 0 (when there is a hierarchy),
-    // r.z and z.r_old with z = x (z[0] = 0), and the flexible-CG decision. z
+    // r.z and z.r_old with z = x, and the flexible-CG decision. z
     // stays in the finest level's x (FP32); enqueue_pass1 reads it there.
     int enqueue_finish(void* state, const double* r0, const double* r1, int mode, Partials part,
                        rb200_trace* trace, cudaStream_t s) const;

@@ -901,8 +901,8 @@ __device__ __forceinline__ void train_block(const MgLevelDev& L, const MgLevelDe
 // ------------------------------------------------------------ flexible-CG passes
 
 // The finest level's last red half-sweep fused with the outer method's
-// preconditioner output: z = x (FP64, z[0] = 0 for the eliminated gauge row),
-// r.z and z.r_old reduced and the flexible-CG decision taken. Without a hierarchy
+// preconditioner output: z = x (FP64; the dots take it up to a constant, which
+// they cannot see, since r sums to zero), r.z and z.r_old reduced and the flexible-CG decision taken. Without a hierarchy
 // (a single level solved densely) z is copied from x.
 __device__ __forceinline__ void finish_red_body(const MgLevelDev& L, int smooth, SolveState* st, const double* r0,
                                                 const double* r1, int mode, Partials part, rb200_trace* trace,
@@ -957,7 +957,7 @@ __device__ __forceinline__ void finish_red_body(const MgLevelDev& L, int smooth,
                 }
                 double zc[4];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) zc[e] = (c0 + e == 0) ? 0.0 : double(f4get(out, e));
+                for (int e = 0; e < 4; ++e) zc[e] = double(f4get(out, e));
                 const double2 r01 = *reinterpret_cast<const double2*>(r + c0);
                 const double2 r23 = *reinterpret_cast<const double2*>(r + c0 + 2);
                 const double rr[4] = {r01.x, r01.y, r23.x, r23.y};
@@ -965,7 +965,6 @@ __device__ __forceinline__ void finish_red_body(const MgLevelDev& L, int smooth,
                 if (mode == MODE_ITER) ld_quad(r_old + c0, ro);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    if (c0 + e == 0) continue;
                     rz.add(rr[e] * zc[e]);
                     if (mode == MODE_ITER) zq.add(zc[e] * ro[e]);
                 }
@@ -981,11 +980,9 @@ __device__ __forceinline__ void finish_red_body(const MgLevelDev& L, int smooth,
             const int ib = i ^ 1;
             if (ib < L.n[0]) {  // the black cell of the pair: its value is final
                 const int c = ib + row;
-                const double zc = c == 0 ? 0.0 : double(L.x[c]);
-                if (c != 0) {
-                    rz.add(r[c] * zc);
-                    if (mode == MODE_ITER) zq.add(zc * r_old[c]);
-                }
+                const double zc = double(L.x[c]);
+                rz.add(r[c] * zc);
+                if (mode == MODE_ITER) zq.add(zc * r_old[c]);
             }
             if (i < L.n[0]) {
                 const int c = i + row;
@@ -994,11 +991,9 @@ __device__ __forceinline__ void finish_red_body(const MgLevelDev& L, int smooth,
                     xv = gs_value<false>(L, L.b[c], i, j, k, c);
                     L.x[c] = xv;
                 }
-                const double zc = c == 0 ? 0.0 : double(xv);
-                if (c != 0) {
-                    rz.add(r[c] * zc);
-                    if (mode == MODE_ITER) zq.add(zc * r_old[c]);
-                }
+                const double zc = double(xv);
+                rz.add(r[c] * zc);
+                if (mode == MODE_ITER) zq.add(zc * r_old[c]);
             }
         }
     }
@@ -1013,7 +1008,7 @@ __device__ __forceinline__ void finish_red_body(const MgLevelDev& L, int smooth,
 // The flexible-CG direction pass of the mixed method (src/pressure.rs:657-668,
 // :720-731): d = z + beta d (d = z after a restart), q = K d, d.q and the
 // decision for alpha; q is not stored (the later passes recompute it). z is read straight from the V-cycle's FP32 output x
-// of the finest level (z = f64(x), z[0] = 0 for the eliminated gauge row), so
+// of the finest level (z = f64(x) - f64(x[0]), mg.hpp), so
 // no FP64 copy of z is stored. One warp per cell row, lanes along x.
 __device__ __forceinline__ void pass1_body(const GridDev& g, const MgLevelDev& L, SolveState* st, double* d0,
                                            double* d1, Partials part, rb200_trace* trace, int kc_len, Span sp) {
@@ -1026,8 +1021,11 @@ __device__ __forceinline__ void pass1_body(const GridDev& g, const MgLevelDev& L
     const double* __restrict__ src = dsel ? d1 : d0;
     double* __restrict__ dst = dsel ? d0 : d1;
     const float* __restrict__ x = L.x;
+    // z = x - x[0]: the V-cycle's output is defined up to a constant, and this
+    // representative keeps d[0] = p[0] = 0 (the gauge)
+    const double x0 = double(x[0]);
     auto dn = [&](int c) -> double {
-        const double zc = c == 0 ? 0.0 : double(x[c]);
+        const double zc = double(x[c]) - x0;
         return fresh ? zc : zc + beta * src[c];
     };
     const int sy = g.n[0], sz = g.n[0] * g.n[1];
@@ -1039,7 +1037,7 @@ __device__ __forceinline__ void pass1_body(const GridDev& g, const MgLevelDev& L
         const int n0 = g.n[0], quads = n0 >> 2;
         auto dn4 = [&](int c0, double (&o)[4]) {
             const float4 xv = *reinterpret_cast<const float4*>(x + c0);
-            const double zc[4] = {c0 == 0 ? 0.0 : double(xv.x), double(xv.y), double(xv.z), double(xv.w)};
+            const double zc[4] = {double(xv.x) - x0, double(xv.y) - x0, double(xv.z) - x0, double(xv.w) - x0};
             if (fresh) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) o[e] = zc[e];
@@ -1091,7 +1089,7 @@ __device__ __forceinline__ void pass1_body(const GridDev& g, const MgLevelDev& L
                     v.yp = yp[e];
                     v.zm = prev[e];
                     v.zp = next[e];
-                    qq[e] = (c0 + e == 0) ? 0.0 : apply_row(g, i0 + e, j, k, v);
+                    qq[e] = apply_row(g, i0 + e, j, k, v);
                 }
                 *reinterpret_cast<double2*>(dst + c0) = make_double2(cur[0], cur[1]);
                 *reinterpret_cast<double2*>(dst + c0 + 2) = make_double2(cur[2], cur[3]);
@@ -1117,7 +1115,7 @@ __device__ __forceinline__ void pass1_body(const GridDev& g, const MgLevelDev& L
             v.yp = j + 1 < g.n[1] ? dn(c + sy) : 0.0;
             v.zm = k > 0 ? dn(c - sz) : 0.0;
             v.zp = k + 1 < g.n[2] ? dn(c + sz) : 0.0;
-            const double qv = c == 0 ? 0.0 : apply_row(g, i, j, k, v);
+            const double qv = apply_row(g, i, j, k, v);
             dst[c] = v.c;
             acc.add(v.c * qv);
         }
@@ -1169,11 +1167,9 @@ __device__ __forceinline__ void update_first_body(const GridDev& g, const MgLeve
                 float4 bq, xq = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    if (c0 + e != 0) {  // the gauge row keeps p[0] = r[0] = 0
-                        pv[e] = pv[e] + alpha * dv[e];
-                        rv[e] = rv[e] - alpha * qv[e];
-                        acc.add(rv[e] * rv[e]);
-                    }
+                    pv[e] = pv[e] + alpha * dv[e];
+                    rv[e] = rv[e] - alpha * qv[e];
+                    acc.add(rv[e] * rv[e]);
                     f4put(bq, e, float(rv[e]));
                 }
 #pragma unroll
@@ -1192,12 +1188,9 @@ __device__ __forceinline__ void update_first_body(const GridDev& g, const MgLeve
         } else {
             for (int i = W.lane; i < n0; i += 32) {
                 const int c = base + i;
-                double rc = r[c];
-                if (c != 0) {
-                    p[c] = p[c] + alpha * d[c];
-                    rc = rc - alpha * kd_at(g, d, i, j, k, c);
-                    acc.add(rc * rc);
-                }
+                p[c] = p[c] + alpha * d[c];
+                const double rc = r[c] - alpha * kd_at(g, d, i, j, k, c);
+                acc.add(rc * rc);
                 r_out[c] = rc;
                 const float b = float(rc);
                 L.b[c] = b;

@@ -296,8 +296,8 @@ __global__ void __launch_bounds__(TILE_THREADS) k_true_residual(GridDev g, Solve
 // ------------------------------------------------------------ multigrid outer passes
 // Flexible CG around the FP32 multigrid preconditioner: q = K d is formed by
 // pass 1 for d.q and recomputed from d where the update and the finish need it
-// (no q vector); the finish pass converts the FP32 V-cycle output to z (FP64,
-// z[0] = 0), reduces r.z and z.r_old and takes the decision with the
+// (no q vector); the finish pass takes the FP32 V-cycle output as z (FP64),
+// reduces r.z and z.r_old and takes the decision with the
 // Polak-Ribiere beta = (z.r - z.r_old) / (z_old.r_old) (tolerant of a
 // preconditioner that is symmetric only up to FP32 rounding). The residual
 // before the update stays available in a second buffer. This update serves
@@ -315,10 +315,6 @@ __global__ void __launch_bounds__(EW) k_mg_update(GridDev g, SolveState* st, dou
     const double* __restrict__ d = st->dsel ? d1 : d0;
     Neu acc;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < g.cells; c += gridDim.x * blockDim.x) {
-        if (c == 0) {
-            r_old[0] = 0.0;
-            continue;
-        }
         int i, j, k;
         cell_coords(g, c, i, j, k);
         p[c] = p[c] + alpha * d[c];

@@ -41,7 +41,7 @@ __device__ __forceinline__ double apply_row(const GridDev& g, int i, int j, int 
 // direction pass, which saves a write and a read of an FP64 vector per
 // iteration. kd_quad takes the four cells c0..c0+3 of row (j, k) of a grid
 // whose rows are a multiple of 4 long (dv: d at the quad), with 16-byte loads
-// of the y and z neighbour rows; kd_at takes one cell. The gauge row's q is 0.
+// of the y and z neighbour rows; kd_at takes one cell.
 __device__ __forceinline__ void ld_quad(const double* __restrict__ a, double (&o)[4]) {
     const double2 lo = *reinterpret_cast<const double2*>(a);
     const double2 hi = *reinterpret_cast<const double2*>(a + 2);
@@ -71,11 +71,10 @@ __device__ __forceinline__ void kd_quad(const GridDev& g, const double* __restri
         v.yp = yp[e];
         v.zm = zm[e];
         v.zp = zp[e];
-        qq[e] = (c0 + e == 0) ? 0.0 : apply_row(g, i0 + e, j, k, v);
+        qq[e] = apply_row(g, i0 + e, j, k, v);
     }
 }
 __device__ __forceinline__ double kd_at(const GridDev& g, const double* __restrict__ d, int i, int j, int k, int c) {
-    if (c == 0) return 0.0;
     const int sy = g.n[0], sz = g.n[0] * g.n[1];
     Neigh v;
     v.c = d[c];
