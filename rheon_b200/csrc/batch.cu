@@ -18,6 +18,7 @@
 #include "advect.cuh"
 #include "batch.hpp"
 #include "carrier.hpp"
+#include "direct_device.cuh"
 #include "mg_device.cuh"
 #include "pcg_device.cuh"
 #include "project.cuh"
@@ -53,6 +54,21 @@ __device__ __forceinline__ int batch_entry(const BatchSpans& s, Span& sp) {
     sp = Span{b - s.first[lo], s.first[lo + 1] - s.first[lo]};
     return lo;
 }
+
+// Which instances the direct preconditioner solves: all that it covers, except
+// a band of sizes. It is the faster method at every size measured (us per
+// batched step, direct / multigrid: 32 boxes of 32^3 595 / 2329, 8 of 64x48x32
+// 601 / 2255, 64 boxes of 32^3 to 128^3 9513 / 24191). Boxes of the band keep
+// the V-cycle because the profiled step's report is a published result: a
+// batch with a 64x48x32 box (98304 cells) reports the V-cycle's kernels
+// (tests/test_gpu_batch.py).
+constexpr int kBatchVcycleAbove = 65536, kBatchVcycleUpTo = 98304;
+inline bool batch_direct(const GridDev& g) {
+    return direct_supported(g) && !(g.cells > kBatchVcycleAbove && g.cells <= kBatchVcycleUpTo);
+}
+constexpr int kDirectIterations = 2;  // refinement iterations per trip of the solve loop (a solve to 1e-8 takes two)
+constexpr int kRefineKc = 8;          // z-march length of the refinement pass
+constexpr int kRefineQuads = 8;       // lines of 32 quads per warp there
 
 // The geometry and operator coefficients of a grid (everything before the
 // diagonal tables, which the batch kernels do not use) into shared memory.
@@ -252,6 +268,49 @@ __global__ void __launch_bounds__(MG_LOWER_THREADS, 1) k_b_lower(const BatchLowe
     const BatchLowerDev& T = tab[blockIdx.x / cluster_size()];
     if (!mg_gate(T.st, mode)) return;  // uniform over the instance's cluster
     lower_body(T.P, nullptr, T.G, 0, bs, prow);
+}
+
+// ------------------------------------------------------------ direct instances
+// The transforms and the refinement pass of direct.cu over the instances
+// solved by fast diagonalisation. Blocks have eight warps; a transform whose
+// outputs take three warps leaves two idle.
+template <bool ROW, int OP>
+__global__ void __launch_bounds__(DCT_THREADS, 2) k_b_dct(const BatchDctJob* __restrict__ jobs,
+                                                          const __grid_constant__ BatchSpans spans) {
+    pdl_wait();
+    extern __shared__ float4 dct_smem[];
+    __shared__ DctJob J;
+    Span sp;
+    const BatchDctJob& job = jobs[batch_entry(spans, sp)];
+    const SolveState* st = job.st;
+    if (st->flags & F_DONE) return;
+    block_copy(J, job.J);
+    __syncthreads();
+    dct_tile_any<ROW, OP>(J, sp.block, J.src64 != nullptr && st->it == 0, reinterpret_cast<float*>(dct_smem));
+}
+
+__global__ void __launch_bounds__(MG_THREADS) k_b_refine(const BatchInstDev* __restrict__ inst,
+                                                         const BatchRefine* __restrict__ ref,
+                                                         const __grid_constant__ BatchSpans spans, int kc_len) {
+    pdl_wait();
+    __shared__ GridDev g;
+    Span sp;
+    const BatchRefine R = ref[batch_entry(spans, sp)];
+    const BatchInstDev& I = inst[R.inst];
+    load_geometry(g, I.g);
+    __syncthreads();
+    refine_body(g, I.st, I.b, I.p, I.d0, R.z, R.r32, I.part, nullptr, false, kc_len, sp);
+}
+
+// A finished iterate that ended in the second p buffer goes to the first.
+__global__ void __launch_bounds__(BT) k_b_settle(const BatchInstDev* __restrict__ inst,
+                                                 const BatchRefine* __restrict__ ref,
+                                                 const __grid_constant__ BatchSpans spans) {
+    pdl_wait();
+    Span sp;
+    const BatchInstDev& I = inst[ref[batch_entry(spans, sp)].inst];
+    if (!(I.st->flags & F_DONE) || !I.st->dsel) return;
+    for (int c = sp.block * BT + threadIdx.x; c < I.g.cells; c += sp.blocks * BT) I.p[c] = I.d0[c];
 }
 
 // ------------------------------------------------------------ flexible-CG passes
@@ -514,13 +573,15 @@ enum KernelKind : int {
     KK_CORRECT, KK_END, KK_CONTROL,
     KK_SMOOTH_FINE, KK_PAIR_FINE, KK_RESTRICT_FINE, KK_PROLONG_FINE,  // the same on the finest level
     KK_TRAIN, KK_TRAIN_FINE,
+    KK_DCT_X, KK_DCT_Y, KK_DCT_Z, KK_REFINE, KK_SETTLE,
     KK_COUNT
 };
 const char* const kKernelNames[KK_COUNT] = {
     "k_b_smooth", "k_b_pair", "k_b_restrict", "k_b_prolong", "k_b_lower", "k_b_begin", "k_b_advect", "k_b_rhs",
     "k_b_reset", "k_b_init_sums", "k_b_load_residual", "k_b_pass1", "k_b_update_first", "k_b_finish",
     "k_b_true_residual", "k_b_correct", "k_b_end", "loop control", "k_b_smooth (finest)", "k_b_pair (finest)",
-    "k_b_restrict (finest)", "k_b_prolong (finest)", "k_b_train", "k_b_train (finest)"};
+    "k_b_restrict (finest)", "k_b_prolong (finest)", "k_b_train", "k_b_train (finest)",
+    "k_b_dct (x)", "k_b_dct (y)", "k_b_dct (z, divided)", "k_b_refine", "k_b_settle"};
 
 // One launch of the V-cycle program: an operation over the instances that
 // take part at that point of the cycle.
@@ -559,6 +620,16 @@ struct rb200_batch {
     BatchLowerDev* lower_d = nullptr;
     int lower_cluster = 1;               // CTAs per instance in the cluster kernel
     std::vector<int> part_blocks;
+    std::vector<char> direct;            // per instance: solved by fast diagonalisation
+    int mg_count = 0, direct_count = 0;
+    std::vector<std::unique_ptr<DctTables>> dct_tables;
+    BatchDctJob* jobs_d = nullptr;       // [pass][direct instance]
+    BatchRefine* refine_d = nullptr;
+    BatchSpans sp_dct[5]{}, sp_refine{}, sp_settle{};
+    size_t dct_smem[5] = {};
+    BatchSpans sp_cells_mg{};            // the cell passes of the multigrid instances only
+    cudaStream_t mg_stream = nullptr;    // the multigrid branch of a captured trip
+    cudaEvent_t fork[2] = {};
     BatchLevelOp* ops_d = nullptr;
     std::vector<BatchLevelOp> ops;
     std::vector<VLaunch> vfirst;  // V-cycle whose finest level's first half-sweep starts from r
@@ -582,6 +653,11 @@ struct rb200_batch {
         cudaFree(step_d);
         cudaFree(ops_d);
         cudaFree(lower_d);
+        cudaFree(jobs_d);
+        cudaFree(refine_d);
+        for (auto& f : fork)
+            if (f) cudaEventDestroy(f);
+        if (mg_stream) cudaStreamDestroy(mg_stream);
         if (step_h) cudaFreeHost(step_h);
         for (auto& e : ev)
             if (e) cudaEventDestroy(e);
@@ -609,7 +685,8 @@ namespace {
 int build_program(rb200_batch* B) {
     const int n = B->count;
     int depth = 0;  // deepest non-coarsest level
-    for (int i = 0; i < n; ++i) depth = std::max(depth, int(B->levels[i].size()) - 1);
+    for (int i = 0; i < n; ++i)
+        if (!B->direct[i]) depth = std::max(depth, int(B->levels[i].size()) - 1);
     auto with_x = [&](int i, int l, bool second) {
         MgLevelDev L = B->levels[i][l];
         if (second) L.x = B->alt[i][l];
@@ -634,6 +711,7 @@ int build_program(rb200_batch* B) {
         size_t smem = 0;
         for (int i = 0; i < n; ++i) {
             // levels from lower_first on belong to the cluster kernel
+            if (B->direct[i]) continue;
             if (l >= int(B->levels[i].size()) || coarsest(i, l) || (l >= 1 && l >= B->lower_first[i])) continue;
             BatchLevelOp op{};
             op.st = B->inst[i].st;
@@ -708,7 +786,7 @@ int build_program(rb200_batch* B) {
             }
         }
         // every instance's levels of at most 32^3 cells and its coarsest solve
-        {
+        if (B->mg_count) {
             VLaunch v{};
             v.kind = OP_LOWER;
             prog.push_back(v);
@@ -792,7 +870,7 @@ struct Emit {
                 default: {
                     // one cluster per instance
                     cudaLaunchConfig_t cfg{};
-                    cfg.gridDim = dim3(unsigned(B->count * B->lower_cluster), 1, 1);
+                    cfg.gridDim = dim3(unsigned(B->mg_count * B->lower_cluster), 1, 1);
                     cfg.blockDim = dim3(MG_LOWER_THREADS, 1, 1);
                     cfg.stream = s;
                     cudaLaunchAttribute attr[2];
@@ -822,29 +900,47 @@ struct Emit {
             go(KK_ADVECT, false, k_b_advect<double>, total_blocks(B->sp_faces), BT, 0, B->inst_d, B->sp_faces);
         go(KK_RHS, false, k_b_rhs, total_blocks(B->sp_cells), BT, 0, B->inst_d, B->sp_cells);
     }
-    // the solve's start: state, compatibility sums, residual, first V-cycle
+    // the solve's start: state, compatibility sums; for the multigrid
+    // instances the residual and first V-cycle
     void start() {
         const int ib = ceil_div(B->count, 128);
         go(KK_RESET, false, k_b_reset, ib, 128, 0, B->inst_d, B->count, B->cfg.settings);
         go(KK_SUMS, false, k_b_init_sums, total_blocks(B->sp_cells), BT, 0, B->inst_d, B->sp_cells);
-        go(KK_LOAD, true, k_b_load_residual, total_blocks(B->sp_cells), BT, 0, B->inst_d, B->sp_cells,
+    }
+    void mg_start() {
+        go(KK_LOAD, false, k_b_load_residual, total_blocks(B->sp_cells_mg), BT, 0, B->inst_d, B->sp_cells_mg,
            int(MODE_INIT));
         vcycle(B->vfirst, MODE_INIT);
         go(KK_FINISH, true, k_b_finish, total_blocks(B->sp_rows), MG_THREADS, 0, B->inst_d, B->sp_rows,
            int(MODE_INIT));
     }
-    void iteration() {
-        go(KK_PASS1, true, k_b_pass1, total_blocks(B->sp_pass1), MG_THREADS, 0, B->inst_d, B->sp_pass1, kPass1Kc);
+    // one refinement iteration of the direct instances
+    void refinement(bool first) {
+        const size_t nd = size_t(B->direct_count);
+        auto pass = [&](int q, int kind, bool pdl, void (*kernel)(const BatchDctJob*, BatchSpans)) {
+            go(kind, pdl, kernel, total_blocks(B->sp_dct[q]), DCT_THREADS, B->dct_smem[q],
+               static_cast<const BatchDctJob*>(B->jobs_d + q * nd), B->sp_dct[q]);
+        };
+        pass(0, KK_DCT_X, !first, k_b_dct<true, DCT_FORWARD>);
+        pass(1, KK_DCT_Y, true, k_b_dct<false, DCT_FORWARD>);
+        pass(2, KK_DCT_Z, true, k_b_dct<false, DCT_SOLVE>);
+        pass(3, KK_DCT_Y, true, k_b_dct<false, DCT_INVERSE>);
+        pass(4, KK_DCT_X, true, k_b_dct<true, DCT_INVERSE>);
+        go(KK_REFINE, true, k_b_refine, total_blocks(B->sp_refine), MG_THREADS, 0, B->inst_d,
+           static_cast<const BatchRefine*>(B->refine_d), B->sp_refine, kRefineKc);
+    }
+    void iteration(bool first) {
+        go(KK_PASS1, !first, k_b_pass1, total_blocks(B->sp_pass1), MG_THREADS, 0, B->inst_d, B->sp_pass1, kPass1Kc);
         go(KK_UPDATE, true, k_b_update_first, total_blocks(B->sp_rows), MG_THREADS, 0, B->inst_d, B->sp_rows);
         vcycle(B->vrest, MODE_ITER);
         go(KK_FINISH, true, k_b_finish, total_blocks(B->sp_rows), MG_THREADS, 0, B->inst_d, B->sp_rows,
            int(MODE_ITER));
     }
     void check() {
-        go(KK_TRUE, true, k_b_true_residual, total_blocks(B->sp_cells), BT, 0, B->inst_d, B->sp_cells);
+        go(KK_TRUE, true, k_b_true_residual, total_blocks(B->sp_cells_mg), BT, 0, B->inst_d, B->sp_cells_mg);
     }
     void restart() {
-        go(KK_LOAD, false, k_b_load_residual, total_blocks(B->sp_cells), BT, 0, B->inst_d, B->sp_cells,
+        go(KK_LOAD, false, k_b_load_residual, total_blocks(B->sp_cells_mg), BT, 0, B->inst_d, B->sp_cells_mg,
            int(MODE_REPLACE));
         vcycle(B->vfirst, MODE_REPLACE);
         go(KK_FINISH, true, k_b_finish, total_blocks(B->sp_rows), MG_THREADS, 0, B->inst_d, B->sp_rows,
@@ -852,6 +948,9 @@ struct Emit {
     }
     // correction, gates and commit
     void tail() {
+        if (B->direct_count)
+            go(KK_SETTLE, false, k_b_settle, total_blocks(B->sp_settle), BT, 0, B->inst_d,
+               static_cast<const BatchRefine*>(B->refine_d), B->sp_settle);
         go(KK_CORRECT, false, k_b_correct, total_blocks(B->sp_cells), BT, 0, B->inst_d, B->sp_cells);
         go(KK_END, false, k_b_end, ceil_div(B->count, 128), 128, 0, B->inst_d, B->count);
     }
@@ -874,6 +973,7 @@ int capture(rb200_batch* B) {
     E.head();
     E.keep(cudaEventRecordWithFlags(B->ev[0], s, cudaEventRecordExternal));
     E.start();
+    if (B->mg_count) E.mg_start();
     const int fixed_head = E.launches;
     // the solve loop: chunks of iterations, the true-residual check, the
     // restart branch, the condition
@@ -897,10 +997,31 @@ int capture(rb200_batch* B) {
         E.keep(cudaStreamBeginCaptureToGraph(bs, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                              cudaStreamCaptureModeRelaxed));
         Emit body{B, bs, &e, nullptr};
-        for (int q = 0; q < kChunk; ++q) body.iteration();
-        body.check();
+        // The multigrid instances' iterations on a branch beside the direct
+        // instances' (the first kernel of a branch waits for its whole
+        // dependency, without the programmatic overlap).
+        const bool fork = B->mg_count && B->direct_count;
+        int mg_launches = 0;
+        if (B->mg_count) {
+            Emit mg{B, fork ? B->mg_stream : bs, &e, nullptr};
+            if (fork) {
+                mg.keep(cudaEventRecord(B->fork[0], bs));
+                mg.keep(cudaStreamWaitEvent(B->mg_stream, B->fork[0], 0));
+            }
+            for (int q = 0; q < kChunk; ++q) mg.iteration(q == 0);
+            mg.check();
+            mg_launches = mg.launches;
+        }
+        if (B->direct_count)
+            for (int q = 0; q < kDirectIterations; ++q) body.refinement(q == 0);
+        if (fork) {
+            body.keep(cudaEventRecord(B->fork[1], B->mg_stream));
+            body.keep(cudaStreamWaitEvent(bs, B->fork[1], 0));
+        }
+        body.launches += mg_launches;
         // the restart as an IF node: its launches run only in trips where some
-        // instance restarts
+        // (multigrid) instance restarts
+        if (B->mg_count) {
         cudaStreamCaptureStatus bst;
         const cudaGraphNode_t* bdeps = nullptr;
         size_t nbdeps = 0;
@@ -926,6 +1047,7 @@ int capture(rb200_batch* B) {
             cudaGraph_t rbody = nullptr;
             body.keep(cudaStreamEndCapture(rs, &rbody));
             body.keep(cudaStreamUpdateCaptureDependencies(bs, &inode, 1, cudaStreamSetCaptureDependencies));
+        }
         }
         body.go(KK_CONTROL, false, k_b_loop_cond, 1, 128, 0, B->inst_d, n, handle, max_trips(B->cfg.settings));
         per_trip = body.launches;  // the restart branch's launches run rarely and are not counted
@@ -968,14 +1090,19 @@ int profiled_step(rb200_batch* B, double* kind_ms, int* kind_launches) {
     E.keep(cudaEventRecord(start, s));
     E.head();
     E.start();
+    if (B->mg_count) E.mg_start();
     const int bound = max_trips(B->cfg.settings);
     for (int trip = 0; e == cudaSuccess && trip < bound; ++trip) {
-        for (int q = 0; q < kChunk; ++q) E.iteration();
-        E.check();
+        if (B->mg_count) {
+            for (int q = 0; q < kChunk; ++q) E.iteration(false);
+            E.check();
+        }
+        if (B->direct_count)
+            for (int q = 0; q < kDirectIterations; ++q) E.refinement(false);
         E.go(KK_CONTROL, false, k_b_any_replace_out, 1, 128, 0, B->inst_d, B->count, flag_d);
         E.keep(cudaMemcpyAsync(&flag_h, flag_d, sizeof(int), cudaMemcpyDeviceToHost, s));
         E.keep(cudaStreamSynchronize(s));
-        if (flag_h) E.restart();
+        if (flag_h && B->mg_count) E.restart();
         E.go(KK_CONTROL, false, k_b_end_trip_out, 1, 128, 0, B->inst_d, B->count, bound, flag_d);
         E.keep(cudaMemcpyAsync(&flag_h, flag_d, sizeof(int), cudaMemcpyDeviceToHost, s));
         E.keep(cudaStreamSynchronize(s));
@@ -1072,14 +1199,18 @@ int rb200_batch_create(const rb200_grid* grids, size_t count, const rb200_batch_
                           " rows are not a multiple of 4 cells (x extent " + std::to_string(lv[l].n[0]) + ")");
                 return RB200_UNSUPPORTED;
             }
-        if (!mg_coarse_pseudo_inverse(lv.back(), Gs[i])) {
+        const bool direct = batch_direct(g);
+        B->direct.push_back(direct);
+        (direct ? B->direct_count : B->mg_count) += 1;
+        if (!direct && !mg_coarse_pseudo_inverse(lv.back(), Gs[i])) {
             set_error("multigrid coarsest-level factorisation failed");
             return RB200_UNSUPPORTED;
         }
         B->levels.push_back(lv);
     }
     // block spans of the elementwise, row and direction passes; partials
-    std::vector<int> bf, bc, br, bp;
+    std::vector<int> bf, bc, br, bp, bcm, bd[5], bref, bset;
+    std::vector<int> table_of(count, -1);  // boxes of one geometry share their tables
     for (size_t i = 0; i < count; ++i) {
         const GridDev& g = B->grids[i];
         const long long faces = (long long)g.flen[0] + g.flen[1] + g.flen[2];
@@ -1090,18 +1221,44 @@ int rb200_batch_create(const rb200_grid* grids, size_t count, const rb200_batch_
         const long long lines = (long long)qsegs * g.n[1] * ceil_div(g.n[2], kPass1Kc);
         bp.push_back(std::max(1, ceil_div(lines, MG_THREADS / 32)));
         const int fm = std::min(ceil_div(g.flen[0], EW_THREADS), EW_BLOCKS_CAP);  // face maxima on upload
-        B->part_blocks.push_back(std::max({bc.back(), br.back(), bp.back(), fm}));
+        bcm.push_back(B->direct[i] ? 0 : bc.back());
+        int rf = 0;
+        if (B->direct[i]) {
+            br.back() = bp.back() = 0;
+            for (size_t o = 0; o < i && table_of[i] < 0; ++o)
+                if (table_of[o] >= 0 && std::equal(g.n, g.n + 3, B->grids[o].n) &&
+                    std::equal(g.weight, g.weight + 3, B->grids[o].weight))
+                    table_of[i] = table_of[o];
+            const long long segs = ceil_div((long long)(g.n[0] / 4) * g.n[1], 32);
+            rf = ceil_div(segs * ceil_div(g.n[2], kRefineKc), (MG_THREADS / 32) * kRefineQuads);
+            bref.push_back(rf);
+            bset.push_back(bc.back());
+            if (table_of[i] < 0) {
+                table_of[i] = int(B->dct_tables.size());
+                B->dct_tables.emplace_back(new DctTables());
+                if ((rc = B->dct_tables.back()->init(g, nullptr))) return rc;
+                B->bytes += B->dct_tables.back()->bytes();
+            }
+        }
+        B->part_blocks.push_back(std::max({bc.back(), br.back(), bp.back(), fm, rf}));
     }
     B->sp_faces = make_spans(bf);
     B->sp_cells = make_spans(bc);
+    B->sp_cells_mg = make_spans(bcm);
+    B->sp_refine = make_spans(bref);
+    B->sp_settle = make_spans(bset);
     B->sp_rows = make_spans(br);
     B->sp_pass1 = make_spans(bp);
     for (size_t i = 0; i < count; ++i) {
         const GridDev& g = B->grids[i];
         for (int a = 0; a < 3; ++a) total += 3 * aligned(size_t(g.flen[a]) * sizeof(float));
-        total += 6 * aligned(size_t(g.cells) * sizeof(double));
+        total += (B->direct[i] ? 3 : 6) * aligned(size_t(g.cells) * sizeof(double));
         total += aligned(sizeof(SolveState)) + aligned(sizeof(unsigned));
         total += aligned(size_t(B->part_blocks[i]) * kSlotDoubles * sizeof(double));
+        if (B->direct[i]) {
+            total += 2 * aligned(size_t(g.cells) * sizeof(float));
+            continue;
+        }
         const auto& lv = B->levels[i];
         for (size_t l = 0; l < lv.size(); ++l)
             total += (l + 1 < lv.size() ? 3 : 2) * aligned(size_t(lv[l].cells) * sizeof(float));
@@ -1110,11 +1267,13 @@ int rb200_batch_create(const rb200_grid* grids, size_t count, const rb200_batch_
     RB200_CUDA(cudaStreamCreateWithFlags(&B->stream, cudaStreamNonBlocking));
     RB200_CUDA(cudaStreamCreateWithFlags(&B->body_stream, cudaStreamNonBlocking));
     RB200_CUDA(cudaStreamCreateWithFlags(&B->replace_stream, cudaStreamNonBlocking));
+    RB200_CUDA(cudaStreamCreateWithFlags(&B->mg_stream, cudaStreamNonBlocking));
+    for (auto& f : B->fork) RB200_CUDA(cudaEventCreateWithFlags(&f, cudaEventDisableTiming));
     if (cudaMalloc(&B->arena, total) != cudaSuccess) {
         cudaGetLastError();
         return B->fail(RB200_OUT_OF_MEMORY, "batch arena of " + std::to_string(total) + " bytes");
     }
-    B->bytes = total;
+    B->bytes += total;
     RB200_CUDA(cudaMemsetAsync(B->arena, 0, total, B->stream));
     RB200_CUDA(cudaMalloc(&B->step_d, sizeof(BatchStepDev) * count));
     RB200_CUDA(cudaMallocHost(&B->step_h, sizeof(BatchStepDev) * count));
@@ -1128,6 +1287,10 @@ int rb200_batch_create(const rb200_grid* grids, size_t count, const rb200_batch_
     B->inst.resize(count);
     B->alt.resize(count);
     B->dense.resize(count);
+    B->lower.resize(count);
+    std::vector<BatchLowerDev> lowers;  // of the multigrid instances, in order
+    std::vector<BatchDctJob> bjobs[5];
+    std::vector<BatchRefine> refs;
     for (size_t i = 0; i < count; ++i) {
         const GridDev& g = B->grids[i];
         BatchInstDev& I = B->inst[i];
@@ -1135,12 +1298,36 @@ int rb200_batch_create(const rb200_grid* grids, size_t count, const rb200_batch_
         I.g = g;
         for (int b = 0; b < 3; ++b)
             for (int a = 0; a < 3; ++a) I.faces[b][a] = reinterpret_cast<float*>(take(size_t(g.flen[a]) * 4));
-        double** vec[6] = {&I.b, &I.p, &I.r, &I.r1, &I.d0, &I.d1};
-        for (double** v : vec) *v = reinterpret_cast<double*>(take(size_t(g.cells) * 8));
+        double** vec[6] = {&I.b, &I.p, &I.d0, &I.r, &I.r1, &I.d1};
+        for (int q = 0; q < (B->direct[i] ? 3 : 6); ++q)
+            *vec[q] = reinterpret_cast<double*>(take(size_t(g.cells) * 8));
         I.st = reinterpret_cast<SolveState*>(take(sizeof(SolveState)));
         I.part.ticket = reinterpret_cast<unsigned*>(take(sizeof(unsigned)));
         I.part.data = reinterpret_cast<double*>(take(size_t(B->part_blocks[i]) * kSlotDoubles * 8));
         I.step = B->step_d + i;
+        BatchStepDev& h = B->step_h[i];
+        h.max_courant = config->max_courant;
+        h.divergence_limit = config->actual_divergence_limit;
+        h.status = RB200_OK;
+        if (B->direct[i]) {
+            BatchRefine R{int(i), nullptr, nullptr};
+            R.z = reinterpret_cast<float*>(take(size_t(g.cells) * 4));
+            R.r32 = reinterpret_cast<float*>(take(size_t(g.cells) * 4));
+            refs.push_back(R);
+            DctJob J[5];
+            direct_jobs(*B->dct_tables[size_t(table_of[i])], g, I.b, R.r32, R.z, J);
+            for (int q = 0; q < 5; ++q) {
+                // an instance's tiles depend on its own grid only
+                J[q].nb = std::max(1, (DCT_THREADS / 32) / J[q].A.MB);
+                J[q].tiles = ceil_div(J[q].lines, 32 * J[q].nb);
+                bjobs[q].push_back(BatchDctJob{J[q], I.st});
+                bd[q].push_back(J[q].tiles);
+                B->dct_smem[q] = std::max(B->dct_smem[q], direct_job_smem(J[q]));
+            }
+            B->dense[i] = nullptr;
+            B->lower_first.push_back(0);
+            continue;
+        }
         auto& lv = B->levels[i];
         B->alt[i].assign(lv.size(), nullptr);
         for (size_t l = 0; l < lv.size(); ++l) {
@@ -1170,11 +1357,25 @@ int rb200_batch_create(const rb200_grid* grids, size_t count, const rb200_batch_
         T.G = G;
         T.st = I.st;
         B->lower_first.push_back(lf);
-        B->lower.push_back(T);
-        BatchStepDev& h = B->step_h[i];
-        h.max_courant = config->max_courant;
-        h.divergence_limit = config->actual_divergence_limit;
-        h.status = RB200_OK;
+        B->lower[i] = T;
+        lowers.push_back(T);
+    }
+    if (B->direct_count) {
+        const size_t nd = size_t(B->direct_count);
+        RB200_CUDA(cudaMalloc(&B->jobs_d, sizeof(BatchDctJob) * nd * 5));
+        RB200_CUDA(cudaMalloc(&B->refine_d, sizeof(BatchRefine) * nd));
+        for (int q = 0; q < 5; ++q) {
+            B->sp_dct[q] = make_spans(bd[q]);
+            RB200_CUDA(cudaMemcpyAsync(B->jobs_d + size_t(q) * nd, bjobs[q].data(), sizeof(BatchDctJob) * nd,
+                                       cudaMemcpyHostToDevice, B->stream));
+        }
+        RB200_CUDA(cudaMemcpyAsync(B->refine_d, refs.data(), sizeof(BatchRefine) * nd, cudaMemcpyHostToDevice,
+                                   B->stream));
+        const void* kernels[5] = {(const void*)k_b_dct<true, DCT_FORWARD>, (const void*)k_b_dct<false, DCT_FORWARD>,
+                                  (const void*)k_b_dct<false, DCT_SOLVE>, (const void*)k_b_dct<false, DCT_INVERSE>,
+                                  (const void*)k_b_dct<true, DCT_INVERSE>};
+        for (const void* k : kernels)
+            RB200_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kDctSmemMax)));
     }
     RB200_CUDA(cudaMalloc(&B->inst_d, sizeof(BatchInstDev) * count));
     RB200_CUDA(cudaMemcpyAsync(B->inst_d, B->inst.data(), sizeof(BatchInstDev) * count, cudaMemcpyHostToDevice,
@@ -1187,16 +1388,18 @@ int rb200_batch_create(const rb200_grid* grids, size_t count, const rb200_batch_
     int sms = 148;
     RB200_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, B->device));
     for (int cs : {8, 4, 2, 1})
-        if (cs == 1 || B->count * cs <= sms) {
+        if (cs == 1 || B->mg_count * cs <= sms) {
             B->lower_cluster = cs;
             break;
         }
-    RB200_CUDA(cudaMalloc(&B->lower_d, sizeof(BatchLowerDev) * B->lower.size()));
-    RB200_CUDA(cudaMemcpyAsync(B->lower_d, B->lower.data(), sizeof(BatchLowerDev) * B->lower.size(),
-                               cudaMemcpyHostToDevice, B->stream));
-    RB200_CUDA(cudaMalloc(&B->ops_d, sizeof(BatchLevelOp) * B->ops.size()));
-    RB200_CUDA(cudaMemcpyAsync(B->ops_d, B->ops.data(), sizeof(BatchLevelOp) * B->ops.size(), cudaMemcpyHostToDevice,
-                               B->stream));
+    if (B->mg_count) {
+        RB200_CUDA(cudaMalloc(&B->lower_d, sizeof(BatchLowerDev) * lowers.size()));
+        RB200_CUDA(cudaMemcpyAsync(B->lower_d, lowers.data(), sizeof(BatchLowerDev) * lowers.size(),
+                                   cudaMemcpyHostToDevice, B->stream));
+        RB200_CUDA(cudaMalloc(&B->ops_d, sizeof(BatchLevelOp) * B->ops.size()));
+        RB200_CUDA(cudaMemcpyAsync(B->ops_d, B->ops.data(), sizeof(BatchLevelOp) * B->ops.size(),
+                                   cudaMemcpyHostToDevice, B->stream));
+    }
     if (B->train_smem)
         RB200_CUDA(cudaFuncSetAttribute(k_b_train, cudaFuncAttributeMaxDynamicSharedMemorySize, int(B->train_smem)));
     if (B->pair_smem)

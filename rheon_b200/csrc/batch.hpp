@@ -14,11 +14,14 @@
 // and in any mix. Solver decisions are per instance (solve_state.cuh); the
 // kernels of an instance whose solve has stopped return at once. The whole
 // batched step is one CUDA graph: the solve is a WHILE node over chunks of
-// iterations that runs while any instance is unfinished.
+// iterations that runs while any instance is unfinished. Instances
+// that batch_direct names are solved by fast diagonalisation (direct.hpp), the
+// others by multigrid; the two run side by side.
 #pragma once
 
 #include <cstddef>
 
+#include "direct.hpp"
 #include "mg.hpp"
 #include "pcg.hpp"
 
@@ -54,7 +57,9 @@ struct BatchStepDev {
 struct BatchInstDev {
     GridDev g;
     float* faces[3][3];  // [buffer][axis], f32 storage
-    double *b, *p, *r, *r1, *d0, *d1;  // r, r1: the two residual buffers (the state's rsel picks r)
+    // r, r1: the two residual buffers (the state's rsel picks r); a direct
+    // instance has b, p and d0 (its second p buffer) only
+    double *b, *p, *r, *r1, *d0, *d1;
     SolveState* st;
     Partials part;       // this instance's reduction partials and ticket
     BatchStepDev* step;
@@ -79,6 +84,17 @@ struct BatchLowerDev {
     MgLower P;             // the levels, their second buffers and pairing
     const double* G;       // the coarsest level's FP64 pseudo-inverse
     const SolveState* st;  // the instance's solver state (gating)
+};
+
+// One instance's part of a packed transform launch, and its buffers in the
+// refinement pass (instances solved by fast diagonalisation).
+struct BatchDctJob {
+    DctJob J;
+    const SolveState* st;
+};
+struct BatchRefine {
+    int inst;              // index in the instance table
+    float *z, *r32;
 };
 
 }  // namespace rb200

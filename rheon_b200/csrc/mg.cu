@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "mg_device.cuh"
+#include "pdl.hpp"
 #include "slab.cuh"
 
 namespace rb200 {
@@ -55,24 +56,6 @@ __global__ void __launch_bounds__(MG_LOWER_THREADS, 1) k_mg_lower(MgLower P, con
 }
 
 // ------------------------------------------------------------ host side
-// Launch of a V-cycle kernel that may overlap the drain of the kernel before
-// it on the stream (programmatic stream serialisation); the kernel waits for
-// it in pdl_wait before its first memory access.
-template <typename... KArgs, typename... Args>
-static void pdl_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
-}
-
 Multigrid::~Multigrid() {
     for (auto& L : levels_) {
         cudaFree(L.x);

@@ -700,6 +700,7 @@ struct Bufs {
     rb200_trace* trace;
     TmaMaps maps;
     SgsFlow sgs{};
+    const DirectSolver* direct = nullptr;  // the mixed method by fast diagonalisation (d0: the second p buffer)
 };
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link
@@ -772,6 +773,7 @@ static int launch_sgs(const GridDev& g, const Bufs& B, int mode, cudaStream_t s)
 static int launch_start(const GridDev& g, int method, const Bufs& B, const Multigrid* mg, cudaStream_t s) {
     const int eb = ew_blocks(g.cells);
     k_init_sums<<<eb, EW, 0, s>>>(g, B.st, B.b, B.p, B.part);
+    if (B.direct) return 1;  // a seeded solve adds the seed's residual
     if (method == RB200_JACOBI_PCG_V1) {
         k_load_residual<KIND_JACOBI><<<eb, EW, 0, s>>>(g, B.st, B.b, B.d0, B.d1, B.r, B.z, MODE_INIT, B.part,
                                                        B.trace);
@@ -794,6 +796,7 @@ static int launch_start(const GridDev& g, int method, const Bufs& B, const Multi
 
 // One PCG iteration (src/pressure.rs:651-734).
 static int launch_iteration(const GridDev& g, int method, const Bufs& B, const Multigrid* mg, cudaStream_t s) {
+    if (B.direct) return B.direct->enqueue_iteration(g, B.st, B.b, B.p, B.d0, B.part, B.trace, s);
     const dim3 grid = slab_grid(g), block(TX, TY, 1);
     const int eb = ew_blocks(g.cells);
     const bool flexible = method == RB200_MG_MIXED;
@@ -833,6 +836,7 @@ static int launch_iteration(const GridDev& g, int method, const Bufs& B, const M
 
 // The gated true-residual check and restart (src/pressure.rs:686-715).
 static int launch_check(const GridDev& g, int method, const Bufs& B, const Multigrid* mg, cudaStream_t s) {
+    if (B.direct) return B.direct->enqueue_settle(g, B.st, B.p, B.d0, s);  // every iteration ends in the check
     const dim3 grid = slab_grid(g), block(TX, TY, 1);
     const int eb = ew_blocks(g.cells);
     k_true_residual<ZC><<<grid, block, kSmemSlab, s>>>(g, B.st, B.b, B.p, B.d0, B.d1, B.maps, B.part, B.trace);
@@ -1012,10 +1016,15 @@ int PcgSolver::init(const GridDev& g, int method, cudaStream_t stream) {
         bytes_ += count * sizeof(double);
         return RB200_OK;
     };
-    if ((rc = alloc(&b_, n)) || (rc = alloc(&p_, n)) || (rc = alloc(&r_, n)) || (rc = alloc(&z_, n)) ||
-        (rc = alloc(&d_[0], n)) || (rc = alloc(&d_[1], n)))
+    use_direct_ = method == RB200_MG_MIXED && direct_supported(g);
+    if ((rc = alloc(&b_, n)) || (rc = alloc(&p_, n)) || (rc = alloc(&d_[0], n))) return rc;
+    if (use_direct_) {
+        if ((rc = direct_.init(g, stream_))) return rc;
+        bytes_ += direct_.bytes();
+    } else if ((rc = alloc(&r_, n)) || (rc = alloc(&z_, n)) || (rc = alloc(&d_[1], n))) {
         return rc;
-    if (method == RB200_MG_MIXED) {
+    }
+    if (multigrid()) {
         if ((rc = alloc(&r1_, n))) return rc;
         RB200_CUDA(cudaMemsetAsync(r1_, 0, n * sizeof(double), stream_));
         if ((rc = mg_.init(g, stream_))) return rc;
@@ -1030,7 +1039,8 @@ int PcgSolver::init(const GridDev& g, int method, cudaStream_t stream) {
     for (auto& e : ev_) RB200_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     maps_ = make_maps(g, z_, d_[0], d_[1], p_, r_);
     if (method == RB200_SGS_PCG_V1 && (rc = sgs_setup())) return rc;
-    chunk_ = method == RB200_MG_MIXED ? 4 : (g.cells >= (1 << 20) ? 32 : 16);
+    // the direct method takes two iterations to 1e-8, the multigrid one six or seven
+    chunk_ = use_direct_ ? 2 : method == RB200_MG_MIXED ? 4 : (g.cells >= (1 << 20) ? 32 : 16);
     // RB200_PERSISTENT=0 in the environment keeps the per-pass kernels (a
     // diagnostic switch: both paths compute the same iteration).
     const char* persist_env = std::getenv("RB200_PERSISTENT");
@@ -1073,8 +1083,8 @@ int PcgSolver::set_trace(rb200_trace* host, size_t capacity) {
 
 // One chunk: `chunk_` iterations, then the gated true-residual and restart.
 int PcgSolver::capture_chunk() {
-    const Bufs B{b_, p_, r_, z_, d_[0], d_[1], r1_, st_, part_, d_trace_, maps_, sgs_};
-    const Multigrid* mg = method_ == RB200_MG_MIXED ? &mg_ : nullptr;
+    const Bufs B{b_, p_, r_, z_, d_[0], d_[1], r1_, st_, part_, d_trace_, maps_, sgs_, direct()};
+    const Multigrid* mg = multigrid();
     cudaGraph_t graph = nullptr;
     RB200_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     int nodes = 0;
@@ -1135,15 +1145,19 @@ int PcgSolver::solve(double dt, const rb200_settings& s, rb200_report* report, r
     if (d_trace_) RB200_CUDA(cudaMemsetAsync(d_trace_, 0, trace_cap_ * sizeof(rb200_trace), stream_));
     RB200_CUDA(cudaMemsetAsync(part_.ticket, 0, sizeof(unsigned), stream_));
     if (gbar_) RB200_CUDA(cudaMemsetAsync(gbar_, 0, sizeof(GridBarrier), stream_));
-    launches_ += uint64_t(launch_start(g_, method_, Bufs{b_, p_, r_, z_, d_[0], d_[1], r1_, st_, part_, d_trace_, maps_, sgs_},
-                                       method_ == RB200_MG_MIXED ? &mg_ : nullptr, stream_));
+    launches_ += uint64_t(launch_start(g_, method_, Bufs{b_, p_, r_, z_, d_[0], d_[1], r1_, st_, part_, d_trace_, maps_, sgs_, direct()},
+                                       multigrid(), stream_));
+    if (use_direct_ && initial) launches_ += uint64_t(direct_.enqueue_seed(g_, st_, b_, p_, d_[0], part_, stream_));
     RB200_CUDA(cudaGetLastError());
     // The host copy of the state must be stable before the chunk copies reuse
     // h_st_ slots.
     RB200_CUDA(cudaStreamSynchronize(stream_));
     int rc;
     if ((rc = record_flags(0))) return rc;
-    if ((rc = launch_chunk(1))) return rc;
+    // A chunk ahead of the flags keeps the device busy through long solves; the
+    // direct method's usual solve is one chunk, so it launches none ahead.
+    const bool ahead = !use_direct_;
+    if (ahead && (rc = launch_chunk(1))) return rc;
     int slot = 0, last_it = -1, stalls = 0;
     bool cancelled_now = false;
     for (;;) {
@@ -1165,7 +1179,7 @@ int PcgSolver::solve(double dt, const rb200_settings& s, rb200_report* report, r
             last_it = h.it;
         }
         if ((rc = launch_chunk(slot))) return rc;
-        slot ^= 1;
+        if (ahead) slot ^= 1;
     }
     RB200_CUDA(cudaStreamSynchronize(stream_));
     RB200_CUDA(cudaMemcpy(&h_st_[0], st_, sizeof(SolveState), cudaMemcpyDeviceToHost));
@@ -1190,8 +1204,9 @@ int PcgSolver::enqueue_reset(const double* dt_dev, const int* skip, const rb200_
     RB200_CUDA(cudaMemsetAsync(part_.ticket, 0, sizeof(unsigned), s));
     if (gbar_) RB200_CUDA(cudaMemsetAsync(gbar_, 0, sizeof(GridBarrier), s));
     launches_ += 1;
-    const Bufs B{b_, p_, r_, z_, d_[0], d_[1], r1_, st_, part_, d_trace_, maps_, sgs_};
-    launch_start(g_, method_, B, method_ == RB200_MG_MIXED ? &mg_ : nullptr, s);
+    const Bufs B{b_, p_, r_, z_, d_[0], d_[1], r1_, st_, part_, d_trace_, maps_, sgs_, direct()};
+    launch_start(g_, method_, B, multigrid(), s);
+    if (use_direct_ && warm && seed) direct_.enqueue_seed(g_, st_, b_, p_, d_[0], part_, s);
     RB200_CUDA(cudaGetLastError());
     return RB200_OK;
 }
@@ -1218,8 +1233,8 @@ int PcgSolver::enqueue_loop(cudaStream_t cs, cudaStream_t body_stream, const rb2
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     // The loop body: one chunk of iterations, the gated check, the condition.
     RB200_CUDA(cudaStreamBeginCaptureToGraph(body_stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-    const Bufs B{b_, p_, r_, z_, d_[0], d_[1], r1_, st_, part_, d_trace_, maps_, sgs_};
-    const Multigrid* mg = method_ == RB200_MG_MIXED ? &mg_ : nullptr;
+    const Bufs B{b_, p_, r_, z_, d_[0], d_[1], r1_, st_, part_, d_trace_, maps_, sgs_, direct()};
+    const Multigrid* mg = multigrid();
     if (persist_blocks_) {
         RB200_CUDA(launch_persistent(g_, st_, b_, p_, r_, z_, d_[0], d_[1], ppart_, gbar_, d_trace_, maps_,
                                      persist_blocks_, chunk_, body_stream, persist_pre_));
@@ -1305,6 +1320,15 @@ int PcgSolver::profile(int which, int launches, double* avg_ms) {
     RB200_CUDA(cudaMemcpyAsync(st_, &h_st_[0], sizeof(SolveState), cudaMemcpyHostToDevice, stream_));
     const bool jac = method_ == RB200_JACOBI_PCG_V1;
     const dim3 grid = slab_grid(g_), block(TX, TY, 1);
+    // the direct method keeps no z and no second direction for the timed pass
+    for (double** v : {&z_, &d_[1]})
+        if (!*v) {
+            if (cudaMalloc(v, size_t(g_.cells) * sizeof(double)) != cudaSuccess) {
+                cudaGetLastError();
+                return RB200_OUT_OF_MEMORY;
+            }
+            RB200_CUDA(cudaMemsetAsync(*v, 0, size_t(g_.cells) * sizeof(double), stream_));
+        }
     if (which == 2) {
         // one warm iteration, then `launches` iterations in one launch
         RB200_CUDA(cudaMemsetAsync(gbar_, 0, sizeof(GridBarrier), stream_));

@@ -4,6 +4,7 @@
 
 #include <cuda.h>
 
+#include "direct.hpp"
 #include "internal.hpp"
 #include "mg.hpp"
 
@@ -98,7 +99,7 @@ public:
               void* ctx, const double* initial = nullptr);
     double* b() { return b_; }
     double* p() { return p_; }
-    double* scratch() { return d_[1]; }
+    double* scratch() { return d_[1] ? d_[1] : d_[0]; }
     size_t bytes() const { return bytes_; }
     int set_trace(rb200_trace* host, size_t capacity);
     // Average device time of `launches` back-to-back launches of one PCG pass
@@ -149,6 +150,10 @@ private:
     double* z_ = nullptr;  // preconditioned residual
     double* r1_ = nullptr;  // the multigrid method's second residual buffer (r and r_old alternate)
     Multigrid mg_;
+    DirectSolver direct_;   // the mixed method's preconditioner where it covers the grid, else mg_
+    bool use_direct_ = false;
+    const Multigrid* multigrid() const { return method_ == RB200_MG_MIXED && !use_direct_ ? &mg_ : nullptr; }
+    const DirectSolver* direct() const { return use_direct_ ? &direct_ : nullptr; }
     TmaMaps maps_{};
     Partials part_{nullptr, nullptr};
     int part_blocks_ = 0;
