@@ -20,6 +20,7 @@
 
 #include "pcg.hpp"
 #include "pcg_device.cuh"
+#include "resident.hpp"
 #include "slab.cuh"
 #include "solve_state.cuh"
 #include "stencil.cuh"
@@ -900,6 +901,7 @@ PcgSolver::~PcgSolver() {
     cudaFree(d_trace_);
     cudaFree(gbar_);
     cudaFree(ppart_);
+    cudaFree(rwords_);
     cudaFree(const_cast<int*>(sgs_.order));
     cudaFree(sgs_.ctl);
     if (h_st_) cudaFreeHost(h_st_);
@@ -1045,7 +1047,26 @@ int PcgSolver::init(const GridDev& g, int method, cudaStream_t stream) {
     // diagnostic switch: both paths compute the same iteration).
     const char* persist_env = std::getenv("RB200_PERSISTENT");
     const bool persist_allowed = !(persist_env && persist_env[0] == '0');
-    if ((method == RB200_JACOBI_PCG_V1 || method == RB200_RBSGS_PCG) && maps_.use && persist_allowed) {
+    // Jacobi-PCG keeps its direction on the chip where every brick of 32 x 16 x 32
+    // cells has an SM (up to 128^3); larger grids stream their vectors through
+    // the persistent kernel. us per iteration, resident / before: 32^3 5.4 / 24
+    // (per-pass kernels), 64^3 7.7 / 12.9, 80x48x45 7.7 / 12.9, 96^3 13.3 / 21.4,
+    // 128^3 22.6 / 34.6.
+    if (method == RB200_JACOBI_PCG_V1 && persist_allowed && (rc = resident_setup(g, &resident_))) return rc;
+    if (resident_.q) {
+        RB200_CUDA(cudaMalloc(&gbar_, sizeof(GridBarrier)));
+        const size_t words = resident_words(resident_);
+        RB200_CUDA(cudaMalloc(&rwords_, words * sizeof(unsigned long long)));
+        bytes_ += words * sizeof(unsigned long long);
+        RB200_CUDA(reset_persistent(stream_));
+        persist_blocks_ = resident_.blocks;
+        if (!persistent_graphs_supported(*this)) {
+            persist_blocks_ = 0;
+            resident_.q = 0;
+        } else {
+            chunk_ = 64;
+        }
+    } else if ((method == RB200_JACOBI_PCG_V1 || method == RB200_RBSGS_PCG) && maps_.use && persist_allowed) {
         persist_pre_ = method == RB200_RBSGS_PCG ? 1 : 0;
         int blocks = 0;
         if ((rc = persistent_setup(g, &blocks))) return rc;
@@ -1061,9 +1082,18 @@ int PcgSolver::init(const GridDev& g, int method, cudaStream_t stream) {
     return capture_chunk();
 }
 
-cudaError_t PcgSolver::launch_persistent_chunk(cudaStream_t s, int budget) {
-    return launch_persistent(g_, st_, b_, p_, r_, z_, d_[0], d_[1], ppart_, gbar_, d_trace_, maps_, persist_blocks_,
+cudaError_t PcgSolver::launch_persistent_chunk(cudaStream_t s, int budget, rb200_trace* trace) {
+    if (resident_.q)
+        return launch_resident(resident_, g_, st_, b_, p_, r_, z_, d_[0], d_[1], rwords_, gbar_, trace, budget, s);
+    return launch_persistent(g_, st_, b_, p_, r_, z_, d_[0], d_[1], ppart_, gbar_, trace, maps_, persist_blocks_,
                              budget, s, persist_pre_);
+}
+
+cudaError_t PcgSolver::reset_persistent(cudaStream_t s) {
+    cudaError_t e = cudaMemsetAsync(gbar_, 0, sizeof(GridBarrier), s);
+    if (e == cudaSuccess && rwords_)
+        e = cudaMemsetAsync(rwords_, 0, resident_words(resident_) * sizeof(unsigned long long), s);
+    return e;
 }
 
 int PcgSolver::set_trace(rb200_trace* host, size_t capacity) {
@@ -1090,8 +1120,7 @@ int PcgSolver::capture_chunk() {
     int nodes = 0;
     cudaError_t launch_err = cudaSuccess;
     if (persist_blocks_) {
-        launch_err = launch_persistent(g_, st_, b_, p_, r_, z_, d_[0], d_[1], ppart_, gbar_, d_trace_, maps_,
-                                       persist_blocks_, chunk_, stream_, persist_pre_);
+        launch_err = launch_persistent_chunk(stream_, chunk_);
         nodes = 1;
     } else {
         for (int q = 0; q < chunk_; ++q) nodes += launch_iteration(g_, method_, B, mg, stream_);
@@ -1144,7 +1173,7 @@ int PcgSolver::solve(double dt, const rb200_settings& s, rb200_report* report, r
     RB200_CUDA(cudaMemcpyAsync(st_, &h_st_[0], sizeof(SolveState), cudaMemcpyHostToDevice, stream_));
     if (d_trace_) RB200_CUDA(cudaMemsetAsync(d_trace_, 0, trace_cap_ * sizeof(rb200_trace), stream_));
     RB200_CUDA(cudaMemsetAsync(part_.ticket, 0, sizeof(unsigned), stream_));
-    if (gbar_) RB200_CUDA(cudaMemsetAsync(gbar_, 0, sizeof(GridBarrier), stream_));
+    if (persist_blocks_) RB200_CUDA(reset_persistent(stream_));
     launches_ += uint64_t(launch_start(g_, method_, Bufs{b_, p_, r_, z_, d_[0], d_[1], r1_, st_, part_, d_trace_, maps_, sgs_, direct()},
                                        multigrid(), stream_));
     if (use_direct_ && initial) launches_ += uint64_t(direct_.enqueue_seed(g_, st_, b_, p_, d_[0], part_, stream_));
@@ -1202,7 +1231,7 @@ int PcgSolver::enqueue_reset(const double* dt_dev, const int* skip, const rb200_
     k_solve_reset<<<1, 1, 0, s>>>(st_, settings, dt_dev, skip, method_ == RB200_MG_MIXED ? 1 : 0,
                                   (warm && seed) ? warm : nullptr);
     RB200_CUDA(cudaMemsetAsync(part_.ticket, 0, sizeof(unsigned), s));
-    if (gbar_) RB200_CUDA(cudaMemsetAsync(gbar_, 0, sizeof(GridBarrier), s));
+    if (persist_blocks_) RB200_CUDA(reset_persistent(s));
     launches_ += 1;
     const Bufs B{b_, p_, r_, z_, d_[0], d_[1], r1_, st_, part_, d_trace_, maps_, sgs_, direct()};
     launch_start(g_, method_, B, multigrid(), s);
@@ -1236,8 +1265,7 @@ int PcgSolver::enqueue_loop(cudaStream_t cs, cudaStream_t body_stream, const rb2
     const Bufs B{b_, p_, r_, z_, d_[0], d_[1], r1_, st_, part_, d_trace_, maps_, sgs_, direct()};
     const Multigrid* mg = multigrid();
     if (persist_blocks_) {
-        RB200_CUDA(launch_persistent(g_, st_, b_, p_, r_, z_, d_[0], d_[1], ppart_, gbar_, d_trace_, maps_,
-                                     persist_blocks_, chunk_, body_stream, persist_pre_));
+        RB200_CUDA(launch_persistent_chunk(body_stream, chunk_));
     } else if (mg) {
         // The multigrid restart (a whole V-cycle) as an IF node after the
         // true-residual check: its launches run only in trips that restart.
@@ -1331,15 +1359,13 @@ int PcgSolver::profile(int which, int launches, double* avg_ms) {
         }
     if (which == 2) {
         // one warm iteration, then `launches` iterations in one launch
-        RB200_CUDA(cudaMemsetAsync(gbar_, 0, sizeof(GridBarrier), stream_));
-        RB200_CUDA(launch_persistent(g_, st_, b_, p_, r_, z_, d_[0], d_[1], ppart_, gbar_, nullptr, maps_,
-                                     persist_blocks_, 1, stream_, persist_pre_));
+        RB200_CUDA(reset_persistent(stream_));
+        RB200_CUDA(launch_persistent_chunk(stream_, 1, nullptr));
         cudaEvent_t a, b;
         RB200_CUDA(cudaEventCreate(&a));
         RB200_CUDA(cudaEventCreate(&b));
         RB200_CUDA(cudaEventRecord(a, stream_));
-        RB200_CUDA(launch_persistent(g_, st_, b_, p_, r_, z_, d_[0], d_[1], ppart_, gbar_, nullptr, maps_,
-                                     persist_blocks_, launches, stream_, persist_pre_));
+        RB200_CUDA(launch_persistent_chunk(stream_, launches, nullptr));
         RB200_CUDA(cudaEventRecord(b, stream_));
         RB200_CUDA(cudaEventSynchronize(b));
         float ms = 0.0f;

@@ -74,6 +74,14 @@ struct SgsFlow {
     int blocks = 0;              // resident blocks of the sweep kernel
 };
 
+// Launch plan of the resident Jacobi-PCG kernel (resident.cu); q = 0: the grid
+// does not fit it.
+struct ResidentPlan {
+    int q = 0;            // cells per thread (a z run)
+    int nbx = 0, nby = 0, blocks = 0;
+    size_t smem = 0;
+};
+
 // Persistent PCG kernel (persist.cu); pre: 0 Jacobi, 1 red-black SGS.
 int persistent_setup(const GridDev& g, int* blocks);
 size_t persistent_partial_doubles(int blocks);
@@ -125,7 +133,10 @@ public:
     // Blocks of the persistent solver kernel (0: the per-pass kernels run).
     int persistent_blocks() const { return persist_blocks_; }
     // One launch of the persistent kernel for at most `budget` iterations.
-    cudaError_t launch_persistent_chunk(cudaStream_t s, int budget);
+    cudaError_t launch_persistent_chunk(cudaStream_t s, int budget) { return launch_persistent_chunk(s, budget, d_trace_); }
+    cudaError_t launch_persistent_chunk(cudaStream_t s, int budget, rb200_trace* trace);
+    // Zeroes the barrier (and the reduction words) before a solve.
+    cudaError_t reset_persistent(cudaStream_t s);
     int persist_pre_ = 0;  // preconditioner of the persistent kernel: 0 Jacobi, 1 red-black SGS
     SolveState* state() { return st_; }
     const GridDev& grid() const { return g_; }
@@ -172,6 +183,8 @@ private:
     GridBarrier* gbar_ = nullptr;
     SgsFlow sgs_{};
     double* ppart_ = nullptr;
+    ResidentPlan resident_{};
+    unsigned long long* rwords_ = nullptr;
 };
 
 // Blocks of the slab passes (reduction partials needed per pass).
