@@ -5,6 +5,8 @@
 // f32 or f64 storage) or float (the mixed-precision path).
 #pragma once
 
+#include <type_traits>
+
 #include "internal.hpp"
 
 namespace rb200 {
@@ -22,23 +24,10 @@ __device__ __forceinline__ R clampd(R x, R lo, R hi) {
 
 // (x - o_d) / h_d correctly rounded, through the reciprocal of h_d and one
 // exact remainder (common.cuh) instead of a division: the same bits.
-template <class R>
-__device__ __forceinline__ R div_h(R r, const GridDev& g, int d);
-template <>
-__device__ __forceinline__ double div_h<double>(double r, const GridDev& g, int d) {
-    return div_diag(r, g.h[d], g.rh[d]);
-}
-template <>
-__device__ __forceinline__ float div_h<float>(float r, const GridDev& g, int d) {
-    return div_f32(r, float(g.h[d]), g.rhf[d]);
-}
+__device__ __forceinline__ double div_h(double r, const GridDev& g, int d) { return div_diag(r, g.h[d], g.rh[d]); }
 
 // The integer value of an integer-valued fq in [0, 2^31).
 __device__ __forceinline__ int cell_of(double fq) { return __double2loint(fq + 0x1p52); }
-__device__ __forceinline__ int cell_of(float fq) {
-    if (fq < 0x1p22f) return __float_as_int(fq + 0x1p23f) - 0x4B000000;
-    return int(fq);
-}
 
 // The scaled coordinate (x - o_d) / h_d of a position after the box clamp of
 // ScalarSampler::sample (src/sampling.rs:74-122). It depends on the position
@@ -48,7 +37,7 @@ __device__ __forceinline__ void scaled_position(const GridDev& g, const R pos[3]
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const R x = clampd<R>(pos[d], R(g.o[d]), R(g.up[d]));
-        xh[d] = div_h<R>(x - R(g.o[d]), g, d);
+        xh[d] = div_h(x - R(g.o[d]), g, d);
     }
 }
 
@@ -212,12 +201,236 @@ __device__ __forceinline__ void face_velocity(const GridDev& g, const Faces<T>& 
     }
 }
 
+// ------------------------------------------------------------ FP32 arithmetic
+// The mixed-precision path of the same scheme, in scaled coordinates
+// (x - o) / h throughout: a face or cell centre is p or p + 1/2 exactly, the
+// departure point x - (dt / h) v is one multiply-add per axis, and no division,
+// origin or second clamp is needed. A lattice is offset by 0 or 1/2 along each
+// axis, so a position has two (cell, fraction) pairs per axis, shared by the
+// three velocity components. Interpolation is nested (1 - t) a + t b in
+// multiply-adds; the stored value is clamped to its corners' range, as the
+// reference's sample is. Bound by L1 gathers (40 per face) and issue, about
+// 350 instructions a face where the FP64-style arithmetic in float spent 1270: at
+// 256^3 1780 us before, 790 now for the velocity (issue slots 73 % busy), 748
+// and 320 for the tracer.
+struct LatticeF {
+    float top, last;  // dims - 1, max(dims - 2, 0)
+};
+
+// The cell below q and the fraction within it, q clamped to [0, top]. The cell
+// is q - 1/2 rounded to nearest (an exact integer may give t = 1 in the cell
+// below it: the same value) and at most `last`, so that its upper neighbour
+// exists. BIG: axes beyond the reach of the rounding constant.
+template <bool BIG>
+__device__ __forceinline__ void lattice_cell(float x, const LatticeF& l, int& lo, float& t) {
+    const float q = fminf(fmaxf(x, 0.0f), l.top);
+    if (BIG) {
+        const float f = fminf(floorf(q), l.last);
+        lo = int(f);
+        t = q - f;
+    } else {
+        constexpr float M = 12582912.0f;  // 1.5 2^23
+        const float f = fminf(((q - 0.5f) + M) - M, l.last);
+        lo = __float_as_int(f + M) - 0x4B400000;
+        t = q - f;
+    }
+}
+
+__device__ __forceinline__ float lerp_f(float t, float a, float b) { return fmaf(t, b, fmaf(-t, a, a)); }
+
+// Trilinear value at cell offset `at` of a lattice with strides s1, s2; sx, sy,
+// sz: the upper neighbours' offsets (0 along a one-point axis). CLAMP: to the
+// range of the eight corners.
+template <class T, bool CLAMP>
+__device__ __forceinline__ float trilinear(const T* __restrict__ f, int at, int sx, int sy, int sz, float tx, float ty,
+                                           float tz) {
+    const T* p0 = f + at;
+    const T* p1 = p0 + sy;
+    const T* p2 = p0 + sz;
+    const T* p3 = p2 + sy;
+    const float a0 = float(__ldg(p0)), b0 = float(__ldg(p0 + sx));
+    const float a1 = float(__ldg(p1)), b1 = float(__ldg(p1 + sx));
+    const float a2 = float(__ldg(p2)), b2 = float(__ldg(p2 + sx));
+    const float a3 = float(__ldg(p3)), b3 = float(__ldg(p3 + sx));
+    float r = lerp_f(tz, lerp_f(ty, lerp_f(tx, a0, b0), lerp_f(tx, a1, b1)),
+                     lerp_f(ty, lerp_f(tx, a2, b2), lerp_f(tx, a3, b3)));
+    if (CLAMP) {
+        const float lo = fminf(fminf(fminf(a0, b0), fminf(a1, b1)), fminf(fminf(a2, b2), fminf(a3, b3)));
+        const float hi = fmaxf(fmaxf(fmaxf(a0, b0), fmaxf(a1, b1)), fmaxf(fmaxf(a2, b2), fmaxf(a3, b3)));
+        // not through fmin/fmax: a NaN stays one
+        if (r < lo) r = lo;
+        if (r > hi) r = hi;
+    }
+    return r;
+}
+
+// Strides and lattices of the box, uniform over the launch.
+struct BoxF {
+    LatticeF face[3], cell[3];  // along axis d: the lattice of axis-d faces, and of every other component
+    int up[3];                  // offset factor of the upper neighbour (0 along a one-cell axis)
+};
+__device__ __forceinline__ BoxF box_f(const GridDev& g) {
+    BoxF b;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        b.face[d] = LatticeF{float(g.n[d]), float(g.n[d] - 1)};
+        b.cell[d] = LatticeF{float(g.n[d] - 1), float(max(g.n[d] - 2, 0))};
+        b.up[d] = g.n[d] > 1 ? 1 : 0;
+    }
+    return b;
+}
+
+// The velocity at scaled position x.
+template <class T, bool BIG>
+__device__ __forceinline__ void velocity_f(const GridDev& g, const BoxF& b, const Faces<T>& vel, const float x[3],
+                                           float out[3]) {
+    int lf[3], lc[3];
+    float tf[3], tc[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        lattice_cell<BIG>(x[d], b.face[d], lf[d], tf[d]);
+        lattice_cell<BIG>(x[d] - 0.5f, b.cell[d], lc[d], tc[d]);
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const int s1 = g.fc[a][0], s2 = g.fc[a][0] * g.fc[a][1];
+        const int lx = a == 0 ? lf[0] : lc[0], ly = a == 1 ? lf[1] : lc[1], lz = a == 2 ? lf[2] : lc[2];
+        const int ux = a == 0 ? 1 : b.up[0], uy = a == 1 ? 1 : b.up[1], uz = a == 2 ? 1 : b.up[2];
+        out[a] = trilinear<T, false>(vel.f[a], lx + s1 * ly + s2 * lz, ux, s1 * uy, s2 * uz, a == 0 ? tf[0] : tc[0],
+                                     a == 1 ? tf[1] : tc[1], a == 2 ? tf[2] : tc[2]);
+    }
+}
+
+// The departure point (scaled) of the scaled position x0 with velocity v0
+// there: midpoint RK2. sc: dt / h per axis.
+template <class T, bool BIG>
+__device__ __forceinline__ void departure_f(const GridDev& g, const BoxF& b, const Faces<T>& vel, const float x0[3],
+                                            const float v0[3], const float sc[3], float x[3], int& flag) {
+    float mid[3], v1[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) mid[d] = fmaf(-0.5f * sc[d], v0[d], x0[d]);
+    if (!isfinite(mid[0] + mid[1] + mid[2])) flag |= VF_ARITH;
+    // the sampler clamps to the lattices, which covers the clamp to the box
+    velocity_f<T, BIG>(g, b, vel, mid, v1);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) x[d] = fmaf(-sc[d], v1[d], x0[d]);
+    if (!isfinite(x[0] + x[1] + x[2])) flag |= VF_ARITH;
+}
+
+// dt / h per axis, rounded once from double, by three threads of the block.
+__device__ __forceinline__ void step_scale(const GridDev& g, double dt, float sc[3]) {
+    __shared__ float s[3];
+    if (threadIdx.x < 3) s[threadIdx.x] = float(dt / g.h[threadIdx.x]);
+    __syncthreads();
+#pragma unroll
+    for (int d = 0; d < 3; ++d) sc[d] = s[d];
+}
+
+// The lower faces of cell (p0, p1, p2) along axis A.
+template <class T, bool BIG, int A>
+__device__ __forceinline__ void advect_face_f(const GridDev& g, const BoxF& b, const Faces<T>& vel, const int p[3],
+                                              const float sc[3], double dt, T* __restrict__ out,
+                                              const float* __restrict__ tracer, double gb, int& flag) {
+    const int s1 = g.fc[A][0], s2 = g.fc[A][0] * g.fc[A][1];
+    const int at = p[0] + s1 * p[1] + s2 * p[2];
+    // the upper wall belongs to the last cell
+    if (p[A] + 1 == g.n[A]) out[at + (A == 0 ? 1 : A == 1 ? s1 : s2)] = T(0);
+    if (p[A] == 0) {
+        out[at] = T(0);
+        return;
+    }
+    float v[3];
+    face_velocity<T, float>(g, vel, p, A, v, flag);
+    float x0[3], x[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) x0[d] = float(p[d]) + (d == A ? 0.0f : 0.5f);
+    departure_f<T, BIG>(g, b, vel, x0, v, sc, x, flag);
+    int lo[3];
+    float t[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) lattice_cell<BIG>(d == A ? x[d] : x[d] - 0.5f, d == A ? b.face[d] : b.cell[d], lo[d], t[d]);
+    const float r = trilinear<T, true>(vel.f[A], lo[0] + s1 * lo[1] + s2 * lo[2], A == 0 ? 1 : b.up[0],
+                                       s1 * (A == 1 ? 1 : b.up[1]), s2 * (A == 2 ? 1 : b.up[2]), t[0], t[1], t[2]);
+    if (!isfinite(r)) flag |= VF_ARITH;
+    T value = T(r);
+    if (A == 1 && tracer != nullptr && gb != 0.0) {
+        // Buoyancy hook (new): interior Y face, after advection, before pressure.
+        const int below = cell_idx(g, p[0], p[1] - 1, p[2]), above = cell_idx(g, p[0], p[1], p[2]);
+        const double c = 0.5 * (double(tracer[below]) + double(tracer[above]));
+        const double forced = double(value) + dt * (gb * c);
+        if (!isfinite(forced)) flag |= VF_ARITH;
+        value = T(forced);
+    }
+    out[at] = value;
+}
+
+template <class T, bool BIG>
+__device__ __forceinline__ void advect_velocity_cells_f(const GridDev& g, const Faces<T>& vel, double dt,
+                                                        const float sc[3], T* ou, T* ov, T* ow,
+                                                        const float* __restrict__ tracer, double gb, int* flags,
+                                                        Span sp) {
+    const BoxF b = box_f(g);
+    int local = 0;
+    for (int c = sp.block * blockDim.x + threadIdx.x; c < g.cells; c += sp.blocks * blockDim.x) {
+        int p[3];
+        cell_coords(g, c, p[0], p[1], p[2]);
+        advect_face_f<T, BIG, 0>(g, b, vel, p, sc, dt, ou, tracer, gb, local);
+        advect_face_f<T, BIG, 1>(g, b, vel, p, sc, dt, ov, tracer, gb, local);
+        advect_face_f<T, BIG, 2>(g, b, vel, p, sc, dt, ow, tracer, gb, local);
+    }
+    if (local) atomicOr(flags, local);
+}
+
+template <class T, bool BIG>
+__device__ __forceinline__ void advect_tracer_cells_f(const GridDev& g, const float* __restrict__ old,
+                                                      const Faces<T>& vel, const float sc[3], float* __restrict__ out,
+                                                      int* flags, Span sp) {
+    const BoxF b = box_f(g);
+    const int s1 = g.n[0], s2 = g.n[0] * g.n[1];
+    int local = 0;
+    for (int c = sp.block * blockDim.x + threadIdx.x; c < g.cells; c += sp.blocks * blockDim.x) {
+        int p[3];
+        cell_coords(g, c, p[0], p[1], p[2]);
+        float x0[3], v[3], x[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            // at a cell centre a component is the mean of the cell's two faces
+            const int f1 = g.fc[d][0], f2 = g.fc[d][0] * g.fc[d][1];
+            const T* f = vel.f[d] + (p[0] + f1 * p[1] + f2 * p[2]);
+            v[d] = 0.5f * float(f[0]) + 0.5f * float(f[d == 0 ? 1 : d == 1 ? f1 : f2]);
+            x0[d] = float(p[d]) + 0.5f;
+        }
+        departure_f<T, BIG>(g, b, vel, x0, v, sc, x, local);
+        int lo[3];
+        float t[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) lattice_cell<BIG>(x[d] - 0.5f, b.cell[d], lo[d], t[d]);
+        const float r = trilinear<float, true>(old, lo[0] + s1 * lo[1] + s2 * lo[2], b.up[0], s1 * b.up[1],
+                                               s2 * b.up[2], t[0], t[1], t[2]);
+        if (!isfinite(r)) local |= VF_ARITH;
+        out[c] = r;
+    }
+    if (local) atomicOr(flags, local);
+}
+
+// Axes that the rounding constant of lattice_cell does not reach.
+__device__ __forceinline__ bool big_axes(const GridDev& g) { return max(max(g.n[0], g.n[1]), g.n[2]) >= (1 << 21); }
+
 // advect_velocity (src/advection.rs:28-68): wall-normal faces are exactly 0,
 // every other face samples its own component at the RK2 departure point.
 template <class T, class R>
 __device__ __forceinline__ void advect_velocity_body(const GridDev& g, const Faces<T>& vel, double dt, T* ou, T* ov,
                                                      T* ow, const float* __restrict__ tracer, double gb, int* flags,
                                                      Span sp) {
+    if constexpr (std::is_same<R, float>::value) {
+        float sc[3];
+        step_scale(g, dt, sc);
+        if (big_axes(g))
+            advect_velocity_cells_f<T, true>(g, vel, dt, sc, ou, ov, ow, tracer, gb, flags, sp);
+        else
+            advect_velocity_cells_f<T, false>(g, vel, dt, sc, ou, ov, ow, tracer, gb, flags, sp);
+        return;
+    }
     const long long total = (long long)g.flen[0] + g.flen[1] + g.flen[2];
     int local = 0;
     for (long long t = sp.block * (long long)blockDim.x + threadIdx.x; t < total;
@@ -248,7 +461,7 @@ __device__ __forceinline__ void advect_velocity_body(const GridDev& g, const Fac
 #pragma unroll
         for (int d = 0; d < 3; ++d) pos[d] = R(g.o[d] + (double(p[d]) + (d == a ? 0.0 : 0.5)) * g.h[d]);
         R dep[3];
-        if (std::is_same<R, float>::value || g.exact_centres) {
+        if (g.exact_centres) {
             R initial[3];
             face_velocity<T, R>(g, vel, p, a, initial, local);
             backtrace_from<T, R>(g, vel, pos, initial, R(dt), dep, local);
@@ -279,6 +492,15 @@ template <class T, class R>
 __device__ __forceinline__ void advect_tracer_body(const GridDev& g, const float* __restrict__ old,
                                                    const Faces<T>& vel, double dt, float* __restrict__ out,
                                                    int* flags, Span sp) {
+    if constexpr (std::is_same<R, float>::value) {
+        float sc[3];
+        step_scale(g, dt, sc);
+        if (big_axes(g))
+            advect_tracer_cells_f<T, true>(g, old, vel, sc, out, flags, sp);
+        else
+            advect_tracer_cells_f<T, false>(g, old, vel, sc, out, flags, sp);
+        return;
+    }
     int local = 0;
     int dims[3] = {g.n[0], g.n[1], g.n[2]};
     R off[3] = {R(0.5), R(0.5), R(0.5)};

@@ -46,7 +46,6 @@ struct GridDev {
     int cells;       // n0*n1*n2
     double h[3];
     double rh[3];    // RN(1/h_d) in double where div_diag may use it, else 0
-    float rhf[3];    // RN(1/f32(h_d)) in float where div_f32 may use it, else 0
     int exact_centres;  // nonzero: every cell and face centre scales exactly (make_grid_dev)
     FastDiv frow[3];    // floor(f / fc[a][0]) for a face index f of axis a
     FastDiv fplane[3];  // floor(f / (fc[a][0] fc[a][1]))
@@ -116,21 +115,6 @@ __device__ __forceinline__ double div_diag_fast(double r, double D, double y) {
 }
 __device__ __forceinline__ double div_diag(double r, double D, double y) {
     if (div_diag_fast_ok(r, y)) return div_diag_fast(r, D, y);
-    return r / D;
-}
-
-// The same correctly rounded quotient r / D in binary32 (Markstein's theorem
-// holds for any binary precision): y = RN(1/D) in float, set only for
-// 2^-60 < D < 2^60; the fast path covers r = +-0 and 2^-60 <= |r| < 2^60, where
-// q stays within (2^-120, 2^120) and the remainder above 2^-84, all normal.
-__device__ __forceinline__ float div_f32(float r, float D, float y) {
-    const unsigned ab = __float_as_uint(r) & 0x7fffffffu;
-    const unsigned e = ab >> 23;  // biased exponent; 67..186: 2^-60 <= |r| < 2^60
-    if (y != 0.0f && (e - 67u <= 119u || ab == 0u)) {
-        const float q = r * y;
-        const float rem = fmaf(-q, D, r);
-        return copysignf(fmaf(rem, y, q), r);
-    }
     return r / D;
 }
 
