@@ -14,8 +14,7 @@ namespace rb200 {
 constexpr int ADV_THREADS = 256;
 
 
-template <class R>
-__device__ __forceinline__ R clampd(R x, R lo, R hi) {
+__device__ __forceinline__ double clampd(double x, double lo, double hi) {
     // f64::clamp: if x < min { min } then if x > max { max }.
     if (x < lo) x = lo;
     if (x > hi) x = hi;
@@ -29,78 +28,67 @@ __device__ __forceinline__ double div_h(double r, const GridDev& g, int d) { ret
 // The integer value of an integer-valued fq in [0, 2^31).
 __device__ __forceinline__ int cell_of(double fq) { return __double2loint(fq + 0x1p52); }
 
-// The scaled coordinate (x - o_d) / h_d of a position after the box clamp of
-// ScalarSampler::sample (src/sampling.rs:74-122). It depends on the position
-// only, so the three components of a velocity sample share it.
-template <class R>
-__device__ __forceinline__ void scaled_position(const GridDev& g, const R pos[3], R xh[3]) {
+// The scaled coordinate (x - o_d) / h_d of a position in the box, of
+// ScalarSampler::sample (src/sampling.rs:74-122; its clamp to the box is done
+// where the position is formed). It depends on the position only, so the three
+// components of a velocity sample share it.
+__device__ __forceinline__ void scaled_position(const GridDev& g, const double pos[3], double xh[3]) {
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const R x = clampd<R>(pos[d], R(g.o[d]), R(g.up[d]));
-        xh[d] = div_h(x - R(g.o[d]), g, d);
-    }
+    for (int d = 0; d < 3; ++d) xh[d] = div_h(pos[d] - g.o[d], g, d);
 }
 
-// ScalarSampler::sample (src/sampling.rs:74-122) in arithmetic type R from
-// the scaled coordinate: q = clamp(xh - offset) per axis, the eight corners
-// weighted ((1 * w_x) * w_y) * w_z in the reference's z, y, x order, the sum
-// clamped to the corners' range. 1 * w_x is w_x exactly, so the products
-// w_x w_y are formed once per (x, y) pair and the corner offsets once per
-// axis; the values and every rounding are the reference's. double reproduces
-// the reference; float is the mixed-precision path.
-template <class T, class R>
-__device__ __forceinline__ R sample_at(const T* __restrict__ values, const int dims[3], const R off[3], const R xh[3],
-                                       int& flag) {
-    int lo[3], hi[3];
-    R t[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        R q = clampd<R>(xh[d] - off[d], R(0), R(dims[d] - 1));
-        if (!isfinite(q)) {
-            flag |= VF_ARITH;
-            q = R(0);
-        }
-        // q >= 0, so floor(q) is its truncation; fq is an integer below 2^31,
-        // exactly R(lo), and lo is read from the mantissa of fq + 2^52 (2^23
-        // in float, below 2^22) instead of by conversion instructions
-        const R fq = trunc(q);
-        lo[d] = cell_of(fq);
-        hi[d] = min(lo[d] + 1, dims[d] - 1);
-        t[d] = q - fq;
-    }
-    const R wx[2] = {R(1) - t[0], t[0]};
-    const R wy[2] = {R(1) - t[1], t[1]};
-    const R wz[2] = {R(1) - t[2], t[2]};
-    const R wxy[2][2] = {{wx[0] * wy[0], wx[1] * wy[0]}, {wx[0] * wy[1], wx[1] * wy[1]}};
-    const int px[2] = {lo[0], hi[0]};
-    const int py[2] = {dims[0] * lo[1], dims[0] * hi[1]};
-    const int plane = dims[0] * dims[1];
-    const int pz[2] = {plane * lo[2], plane * hi[2]};
-    R result = R(0);
-    R minimum = R(CUDART_INF);
-    R maximum = R(-CUDART_INF);
+// The cell and fraction of a scaled coordinate on a lattice of top + 1 points:
+// q = clamp(x, 0, top), its floor (q >= 0: the truncation, an integer below
+// 2^31 read from the mantissa of fq + 2^52) and the rest.
+struct Lattice {
+    int lo, hi;
+    double t;
+};
+__device__ __forceinline__ Lattice lattice(double x, int top) {
+    const double q = clampd(x, 0.0, double(top));
+    const double fq = trunc(q);
+    Lattice l;
+    l.lo = cell_of(fq);
+    l.hi = min(l.lo + 1, top);
+    l.t = q - fq;
+    return l;
+}
+
+// ScalarSampler::sample (src/sampling.rs:74-122) from the lattice cells of the
+// three axes: the eight corners weighted ((1 * w_x) * w_y) * w_z in the
+// reference's z, y, x order, the sum clamped to the corners' range. 1 * w_x is
+// w_x exactly, so the products w_x w_y are formed once per (x, y) pair; the
+// values and every rounding are the reference's. Minimum and maximum are plain
+// comparisons (in float for f32 values): the fields are finite.
+template <class T>
+__device__ __forceinline__ double sample_at(const T* __restrict__ values, const Lattice& X, const Lattice& Y,
+                                            const Lattice& Z, int s1, int s2) {
+    const double wx[2] = {1.0 - X.t, X.t};
+    const double wy[2] = {1.0 - Y.t, Y.t};
+    const double wz[2] = {1.0 - Z.t, Z.t};
+    const double wxy[2][2] = {{wx[0] * wy[0], wx[1] * wy[0]}, {wx[0] * wy[1], wx[1] * wy[1]}};
+    const int px[2] = {X.lo, X.hi};
+    const int py[2] = {s1 * Y.lo, s1 * Y.hi};
+    const int pz[2] = {s2 * Z.lo, s2 * Z.hi};
+    double result = 0.0;
+    T minimum{}, maximum{};
 #pragma unroll
     for (int z = 0; z < 2; ++z)
 #pragma unroll
         for (int y = 0; y < 2; ++y)
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
-                const R weight = wxy[y][x] * wz[z];
-                const R value = R(__ldg(values + (px[x] + py[y] + pz[z])));
-                minimum = fmin(minimum, value);
-                maximum = fmax(maximum, value);
-                result += weight * value;
+                const double weight = wxy[y][x] * wz[z];
+                const T value = __ldg(values + (px[x] + py[y] + pz[z]));
+                if (x + y + z == 0) {
+                    minimum = maximum = value;
+                } else {
+                    minimum = value < minimum ? value : minimum;
+                    maximum = value > maximum ? value : maximum;
+                }
+                result += weight * double(value);
             }
-    if (!isfinite(result)) flag |= VF_ARITH;
-    return clampd<R>(result, minimum, maximum);
-}
-
-template <class T, class R>
-__device__ __forceinline__ R sample(const GridDev& g, const T* __restrict__ values, const int dims[3], const R off[3],
-                                    const R pos[3], int& flag) {
-    R xh[3];
-    scaled_position<R>(g, pos, xh);
-    return sample_at<T, R>(values, dims, off, xh, flag);
+    return clampd(result, double(minimum), double(maximum));
 }
 
 template <class T>
@@ -108,59 +96,60 @@ struct Faces {
     const T* f[3];
 };
 
-template <class R>
-__device__ __forceinline__ void face_geometry(const GridDev& g, int a, int dims[3], R off[3]) {
+// The velocity at a position in the box. A component's lattice has n + 1
+// points along its own axis and n along the others, where it is offset by 1/2:
+// two lattice cells per axis serve the three components.
+template <class T>
+__device__ __forceinline__ void velocity_sample(const GridDev& g, const Faces<T>& vel, const double pos[3],
+                                                double out[3]) {
+    double xh[3];
+    scaled_position(g, pos, xh);
+    Lattice own[3], off[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        dims[d] = g.fc[a][d];
-        off[d] = d == a ? R(0) : R(0.5);
+        own[d] = lattice(xh[d], g.n[d]);
+        off[d] = lattice(xh[d] - 0.5, g.n[d] - 1);
     }
-}
-
-template <class T, class R>
-__device__ __forceinline__ void velocity_sample(const GridDev& g, const Faces<T>& vel, const R pos[3], R out[3],
-                                                int& flag) {
-    R xh[3];
-    scaled_position<R>(g, pos, xh);
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        int dims[3];
-        R off[3];
-        face_geometry<R>(g, a, dims, off);
-        out[a] = sample_at<T, R>(vel.f[a], dims, off, xh, flag);
-    }
+    for (int a = 0; a < 3; ++a)
+        out[a] = sample_at<T>(vel.f[a], a == 0 ? own[0] : off[0], a == 1 ? own[1] : off[1], a == 2 ? own[2] : off[2],
+                              g.fc[a][0], g.fc[a][0] * g.fc[a][1]);
 }
 
-// VelocitySampler::departure (src/sampling.rs:160-175).
-template <class R>
-__device__ __forceinline__ void departure(const GridDev& g, const R pos[3], const R vel[3], R dt, R out[3],
-                                          int& flag) {
+// VelocitySampler::departure (src/sampling.rs:160-175). A value that is not
+// finite is flagged (the step or call fails) and replaced, so that the samples
+// stay in range.
+__device__ __forceinline__ void departure(const GridDev& g, const double pos[3], const double vel[3], double dt,
+                                          double out[3], int& flag) {
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        R value = pos[d] - dt * vel[d];
-        if (!isfinite(value)) flag |= VF_ARITH;
-        out[d] = clampd<R>(value, R(g.o[d]), R(g.up[d]));
+        double value = pos[d] - dt * vel[d];
+        if (!isfinite(value)) {
+            flag |= VF_ARITH;
+            value = g.o[d];
+        }
+        out[d] = clampd(value, g.o[d], g.up[d]);
     }
 }
 
 // The second half of VelocitySampler::backtrace (src/sampling.rs:151-159),
 // midpoint RK2, from the velocity at the start point.
-template <class T, class R>
-__device__ __forceinline__ void backtrace_from(const GridDev& g, const Faces<T>& vel, const R pos[3],
-                                               const R initial[3], R dt, R out[3], int& flag) {
-    R mid[3], v1[3];
-    departure<R>(g, pos, initial, R(0.5) * dt, mid, flag);
-    velocity_sample<T, R>(g, vel, mid, v1, flag);
-    departure<R>(g, pos, v1, dt, out, flag);
+template <class T>
+__device__ __forceinline__ void backtrace_from(const GridDev& g, const Faces<T>& vel, const double pos[3],
+                                               const double initial[3], double dt, double out[3], int& flag) {
+    double mid[3], v1[3];
+    departure(g, pos, initial, 0.5 * dt, mid, flag);
+    velocity_sample<T>(g, vel, mid, v1);
+    departure(g, pos, v1, dt, out, flag);
 }
 
 // VelocitySampler::backtrace (src/sampling.rs:151-159): midpoint RK2.
-template <class T, class R>
-__device__ __forceinline__ void backtrace(const GridDev& g, const Faces<T>& vel, const R pos[3], R dt, R out[3],
-                                          int& flag) {
-    R initial[3];
-    velocity_sample<T, R>(g, vel, pos, initial, flag);
-    backtrace_from<T, R>(g, vel, pos, initial, dt, out, flag);
+template <class T>
+__device__ __forceinline__ void backtrace(const GridDev& g, const Faces<T>& vel, const double pos[3], double dt,
+                                          double out[3], int& flag) {
+    double initial[3];
+    velocity_sample<T>(g, vel, pos, initial);
+    backtrace_from<T>(g, vel, pos, initial, dt, out, flag);
 }
 
 // The velocity at the centre of face p of axis a. There the sampler's
@@ -416,8 +405,56 @@ __device__ __forceinline__ void advect_tracer_cells_f(const GridDev& g, const fl
 // Axes that the rounding constant of lattice_cell does not reach.
 __device__ __forceinline__ bool big_axes(const GridDev& g) { return max(max(g.n[0], g.n[1]), g.n[2]) >= (1 << 21); }
 
+// ------------------------------------------------------------ FP64 arithmetic
+// The lower face of cell p along axis A (and the upper wall of the last cell).
+template <class T, int A>
+__device__ __forceinline__ void advect_face_d(const GridDev& g, const Faces<T>& vel, const int p[3], double dt,
+                                              T* __restrict__ out, const float* __restrict__ tracer, double gb,
+                                              int& flag) {
+    const int s1 = g.fc[A][0], s2 = g.fc[A][0] * g.fc[A][1];
+    const int f = p[0] + s1 * p[1] + s2 * p[2];
+    if (p[A] + 1 == g.n[A]) out[f + (A == 0 ? 1 : A == 1 ? s1 : s2)] = T(0);
+    if (p[A] == 0) {
+        out[f] = T(0);
+        return;
+    }
+    double pos[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) pos[d] = g.o[d] + (double(p[d]) + (d == A ? 0.0 : 0.5)) * g.h[d];
+    double dep[3], xh[3];
+    if (g.exact_centres) {
+        double initial[3];
+        face_velocity<T, double>(g, vel, p, A, initial, flag);
+        backtrace_from<T>(g, vel, pos, initial, dt, dep, flag);
+    } else {
+        backtrace<T>(g, vel, pos, dt, dep, flag);
+    }
+    scaled_position(g, dep, xh);
+    Lattice at[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) at[d] = lattice(d == A ? xh[d] : xh[d] - 0.5, d == A ? g.n[d] : g.n[d] - 1);
+    const double sampled = sample_at<T>(vel.f[A], at[0], at[1], at[2], s1, s2);
+    if (!isfinite(sampled)) flag |= VF_ARITH;
+    T value = T(sampled);
+    if (A == 1 && tracer != nullptr && gb != 0.0) {
+        // Buoyancy hook (new): interior Y face, after advection, before pressure.
+        const int below = cell_idx(g, p[0], p[1] - 1, p[2]), above = cell_idx(g, p[0], p[1], p[2]);
+        const double c = 0.5 * (double(tracer[below]) + double(tracer[above]));
+        const double forced = double(value) + dt * (gb * c);
+        if (!isfinite(forced)) flag |= VF_ARITH;
+        value = T(forced);
+    }
+    out[f] = value;
+}
+
 // advect_velocity (src/advection.rs:28-68): wall-normal faces are exactly 0,
-// every other face samples its own component at the RK2 departure point.
+// every other face samples its own component at the RK2 departure point. A
+// thread advects the lower faces of a cell, axis by axis, so that an axis is a
+// constant in the code (one face a thread, of whichever axis, kept its
+// per-axis values in local memory). Bound by issue and the FP64 pipe, about 320
+// operations a face: 128^3 in f64 227 us (108 us of FP64 issue; 417 us with nine
+// lattice cells a sample instead of six, clamps and finite tests repeated per
+// component, and fmin and fmax).
 template <class T, class R>
 __device__ __forceinline__ void advect_velocity_body(const GridDev& g, const Faces<T>& vel, double dt, T* ou, T* ov,
                                                      T* ow, const float* __restrict__ tracer, double gb, int* flags,
@@ -429,61 +466,17 @@ __device__ __forceinline__ void advect_velocity_body(const GridDev& g, const Fac
             advect_velocity_cells_f<T, true>(g, vel, dt, sc, ou, ov, ow, tracer, gb, flags, sp);
         else
             advect_velocity_cells_f<T, false>(g, vel, dt, sc, ou, ov, ow, tracer, gb, flags, sp);
-        return;
+    } else {
+        int local = 0;
+        for (int c = sp.block * blockDim.x + threadIdx.x; c < g.cells; c += sp.blocks * blockDim.x) {
+            int p[3];
+            cell_coords(g, c, p[0], p[1], p[2]);
+            advect_face_d<T, 0>(g, vel, p, dt, ou, tracer, gb, local);
+            advect_face_d<T, 1>(g, vel, p, dt, ov, tracer, gb, local);
+            advect_face_d<T, 2>(g, vel, p, dt, ow, tracer, gb, local);
+        }
+        if (local) atomicOr(flags, local);
     }
-    const long long total = (long long)g.flen[0] + g.flen[1] + g.flen[2];
-    int local = 0;
-    for (long long t = sp.block * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)sp.blocks * blockDim.x) {
-        int a = 0;
-        long long f = t;
-        if (f >= g.flen[0]) {
-            f -= g.flen[0];
-            a = 1;
-            if (f >= g.flen[1]) {
-                f -= g.flen[1];
-                a = 2;
-            }
-        }
-        // face coordinates by multiply-shift (face indices of one axis fit 31 bits)
-        const int fi = int(f);
-        int p[3];
-        p[2] = fast_div(fi, g.fplane[a]);
-        const int in_plane = fi - p[2] * (g.fc[a][0] * g.fc[a][1]);
-        p[1] = fast_div(in_plane, g.frow[a]);
-        p[0] = in_plane - p[1] * g.fc[a][0];
-        T* dst = a == 0 ? ou : (a == 1 ? ov : ow);
-        if (p[a] == 0 || p[a] + 1 == g.fc[a][a]) {
-            dst[f] = T(0);
-            continue;
-        }
-        R pos[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) pos[d] = R(g.o[d] + (double(p[d]) + (d == a ? 0.0 : 0.5)) * g.h[d]);
-        R dep[3];
-        if (g.exact_centres) {
-            R initial[3];
-            face_velocity<T, R>(g, vel, p, a, initial, local);
-            backtrace_from<T, R>(g, vel, pos, initial, R(dt), dep, local);
-        } else {
-            backtrace<T, R>(g, vel, pos, R(dt), dep, local);
-        }
-        int dims[3];
-        R off[3];
-        face_geometry<R>(g, a, dims, off);
-        T value = T(sample<T, R>(g, vel.f[a], dims, off, dep, local));
-        if (a == 1 && tracer != nullptr && gb != 0.0) {
-            // Buoyancy hook (new): interior Y face, after advection, before pressure.
-            int below = cell_idx(g, p[0], p[1] - 1, p[2]);
-            int above = cell_idx(g, p[0], p[1], p[2]);
-            double c = 0.5 * (double(tracer[below]) + double(tracer[above]));
-            double forced = double(value) + dt * (gb * c);
-            if (!isfinite(forced)) local |= VF_ARITH;
-            value = T(forced);
-        }
-        dst[f] = value;
-    }
-    if (local) atomicOr(flags, local);
 }
 
 // advect_tracer (src/advection.rs:72-102), evaluated densely; the reference's
@@ -502,17 +495,20 @@ __device__ __forceinline__ void advect_tracer_body(const GridDev& g, const float
         return;
     }
     int local = 0;
-    int dims[3] = {g.n[0], g.n[1], g.n[2]};
-    R off[3] = {R(0.5), R(0.5), R(0.5)};
     for (int c = sp.block * blockDim.x + threadIdx.x; c < g.cells; c += sp.blocks * blockDim.x) {
         int p[3];
         cell_coords(g, c, p[0], p[1], p[2]);
-        R pos[3];
+        double pos[3], dep[3], xh[3];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) pos[d] = R(g.o[d] + (double(p[d]) + 0.5) * g.h[d]);
-        R dep[3];
-        backtrace<T, R>(g, vel, pos, R(dt), dep, local);
-        out[c] = float(sample<float, R>(g, old, dims, off, dep, local));
+        for (int d = 0; d < 3; ++d) pos[d] = g.o[d] + (double(p[d]) + 0.5) * g.h[d];
+        backtrace<T>(g, vel, pos, dt, dep, local);
+        scaled_position(g, dep, xh);
+        Lattice at[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) at[d] = lattice(xh[d] - 0.5, g.n[d] - 1);
+        const double sampled = sample_at<float>(old, at[0], at[1], at[2], g.n[0], g.n[0] * g.n[1]);
+        if (!isfinite(sampled)) local |= VF_ARITH;
+        out[c] = float(sampled);
     }
     if (local) atomicOr(flags, local);
 }
