@@ -179,11 +179,17 @@ int launch_validate_faces(const GridDev& g, const T* u, const T* v, const T* w, 
 template <class T>
 int launch_build_rhs(const GridDev& g, const T* u, const T* v, const T* w, double dt, double* out,
                      int* flags, cudaStream_t s);
+// build_rhs with the validation of launch_validate_faces in the same pass.
+template <class T>
+int launch_build_rhs_checked(const GridDev& g, const T* u, const T* v, const T* w, double dt, double* out, int* flags,
+                             cudaStream_t s);
+// The divergence; validates the faces in the same pass.
 template <class T>
 int launch_divergence(const GridDev& g, const T* u, const T* v, const T* w, double* out,
                       int* flags, cudaStream_t s);
+// In place; nothing is written when *gate (device) is nonzero.
 template <class T>
-int launch_correct(const GridDev& g, const double* p, double dt, T* u, T* v, T* w, int* flags,
+int launch_correct(const GridDev& g, const double* p, double dt, T* u, T* v, T* w, const int* gate, int* flags,
                    cudaStream_t s);
 
 // Fused projection epilogue of the resident step: corrected faces are written
@@ -208,9 +214,11 @@ int partials_blocks_needed(const GridDev& g);
 template <class T>
 int launch_advect_velocity(const GridDev& g, const T* u, const T* v, const T* w, double dt,
                            T* ou, T* ov, T* ow, const float* tracer, double gb, int* flags,
-                           cudaStream_t s, bool fp32_math = false);
+                           cudaStream_t s, bool fp32_math = false, const int* gate = nullptr);
+// gate (device, or nullptr): nothing is written when it holds VF_NONFINITE.
 template <class T>
 int launch_advect_tracer(const GridDev& g, const float* old, const T* u, const T* v, const T* w,
-                         double dt, float* out, int* flags, cudaStream_t s, bool fp32_math = false);
+                         double dt, float* out, int* flags, cudaStream_t s, bool fp32_math = false,
+                         const int* gate = nullptr);
 
 }  // namespace rb200

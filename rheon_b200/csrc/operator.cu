@@ -39,6 +39,14 @@ int launch_apply_full(const GridDev& g, const double* p, double* out, int* flags
     return RB200_OK;
 }
 
+// The coordinates of face f of axis a by multiply-shift.
+__device__ __forceinline__ void face_coords(const GridDev& g, int a, int f, int& i, int& j, int& k) {
+    k = fast_div(f, g.fplane[a]);
+    const int in_plane = f - k * (g.fc[a][0] * g.fc[a][1]);
+    j = fast_div(in_plane, g.frow[a]);
+    i = in_plane - j * g.fc[a][0];
+}
+
 // ------------------------------------------------------------ finiteness
 // validate_cells (src/operator.rs:840-848): every value finite.
 __global__ void k_check_finite(const double* __restrict__ x, int n, int* flags) {
@@ -76,9 +84,8 @@ __global__ void k_validate_faces(GridDev g, const T* __restrict__ u, const T* __
         const T* src = a == 0 ? u : (a == 1 ? v : w);
         T x = src[f];
         if (!isfinite(double(x))) local |= VF_NONFINITE;
-        int fi = int(f % g.fc[a][0]);
-        int fj = int((f / g.fc[a][0]) % g.fc[a][1]);
-        int fk = int(f / ((long long)g.fc[a][0] * g.fc[a][1]));
+        int fi, fj, fk;
+        face_coords(g, a, int(f), fi, fj, fk);
         if (is_wall_face(g, a, fi, fj, fk) && x != T(0)) local |= VF_WALL;
     }
     if (local) atomicOr(flags, local);
@@ -94,33 +101,46 @@ int launch_validate_faces(const GridDev& g, const T* u, const T* v, const T* w, 
 }
 
 // ------------------------------------------------------------ build_rhs
-template <class T>
+template <class T, bool CHECK>
 __global__ void k_build_rhs(GridDev g, const T* __restrict__ u, const T* __restrict__ v, const T* __restrict__ w,
                             double dt, double* __restrict__ out, int* flags) {
-    build_rhs_body<T>(g, u, v, w, dt, out, flags, whole_launch());
+    build_rhs_body<T, CHECK>(g, u, v, w, dt, out, flags, whole_launch());
 }
 
 template <class T>
 int launch_build_rhs(const GridDev& g, const T* u, const T* v, const T* w, double dt, double* out,
                      int* flags, cudaStream_t s) {
-    k_build_rhs<T><<<ew_blocks(g.cells), EW_THREADS, 0, s>>>(g, u, v, w, dt, out, flags);
+    k_build_rhs<T, false><<<ew_blocks(g.cells), EW_THREADS, 0, s>>>(g, u, v, w, dt, out, flags);
     RB200_CUDA(cudaGetLastError());
     return RB200_OK;
 }
 
 template <class T>
+int launch_build_rhs_checked(const GridDev& g, const T* u, const T* v, const T* w, double dt, double* out, int* flags,
+                             cudaStream_t s) {
+    k_build_rhs<T, true><<<ew_blocks(g.cells), EW_THREADS, 0, s>>>(g, u, v, w, dt, out, flags);
+    RB200_CUDA(cudaGetLastError());
+    return RB200_OK;
+}
+
+// Validates the faces on the way, as build_rhs does.
+template <class T>
 __global__ void k_divergence(GridDev g, const T* __restrict__ u, const T* __restrict__ v,
                              const T* __restrict__ w, double* __restrict__ out, int* flags) {
+    int local = 0;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < g.cells; c += gridDim.x * blockDim.x) {
         int i, j, k;
         cell_coords(g, c, i, j, k);
-        double value = cell_divergence<T>(
-            g, double(u[face_idx(g, 0, i, j, k)]), double(u[face_idx(g, 0, i + 1, j, k)]),
-            double(v[face_idx(g, 1, i, j, k)]), double(v[face_idx(g, 1, i, j + 1, k)]),
-            double(w[face_idx(g, 2, i, j, k)]), double(w[face_idx(g, 2, i, j, k + 1)]));
-        if (!isfinite(value)) atomicOr(flags, VF_ARITH);
+        const double lo[3] = {double(u[face_idx(g, 0, i, j, k)]), double(v[face_idx(g, 1, i, j, k)]),
+                              double(w[face_idx(g, 2, i, j, k)])};
+        const double hi[3] = {double(u[face_idx(g, 0, i + 1, j, k)]), double(v[face_idx(g, 1, i, j + 1, k)]),
+                              double(w[face_idx(g, 2, i, j, k + 1)])};
+        local |= face_checks(g, i, j, k, lo, hi);
+        double value = cell_divergence<T>(g, lo[0], hi[0], lo[1], hi[1], lo[2], hi[2]);
+        if (!isfinite(value)) local |= VF_ARITH;
         out[c] = value;
     }
+    if (local) atomicOr(flags, local);
 }
 
 template <class T>
@@ -132,8 +152,9 @@ int launch_divergence(const GridDev& g, const T* u, const T* v, const T* w, doub
 }
 
 template <class T>
-__global__ void k_correct(GridDev g, const double* __restrict__ p, double dt, T* u, T* v, T* w,
+__global__ void k_correct(GridDev g, const double* __restrict__ p, double dt, T* u, T* v, T* w, const int* gate,
                           int* flags) {
+    if (*gate) return;  // the inputs failed their checks: the faces stay
     const long long total = (long long)g.flen[0] + g.flen[1] + g.flen[2];
     const int s[3] = {1, g.n[0], g.n[0] * g.n[1]};
     int local = 0;
@@ -149,9 +170,8 @@ __global__ void k_correct(GridDev g, const double* __restrict__ p, double dt, T*
                 a = 2;
             }
         }
-        int fi = int(f % g.fc[a][0]);
-        int fj = int((f / g.fc[a][0]) % g.fc[a][1]);
-        int fk = int(f / ((long long)g.fc[a][0] * g.fc[a][1]));
+        int fi, fj, fk;
+        face_coords(g, a, int(f), fi, fj, fk);
         if (is_wall_face(g, a, fi, fj, fk)) continue;
         T* dst = a == 0 ? u : (a == 1 ? v : w);
         int c = cell_idx(g, fi, fj, fk);
@@ -161,10 +181,10 @@ __global__ void k_correct(GridDev g, const double* __restrict__ p, double dt, T*
 }
 
 template <class T>
-int launch_correct(const GridDev& g, const double* p, double dt, T* u, T* v, T* w, int* flags,
+int launch_correct(const GridDev& g, const double* p, double dt, T* u, T* v, T* w, const int* gate, int* flags,
                    cudaStream_t s) {
     long long total = (long long)g.flen[0] + g.flen[1] + g.flen[2];
-    k_correct<T><<<ew_blocks(total), EW_THREADS, 0, s>>>(g, p, dt, u, v, w, flags);
+    k_correct<T><<<ew_blocks(total), EW_THREADS, 0, s>>>(g, p, dt, u, v, w, gate, flags);
     RB200_CUDA(cudaGetLastError());
     return RB200_OK;
 }
@@ -252,9 +272,8 @@ __global__ void k_projection_witness(GridDev g, const double* __restrict__ p, do
         }
         const T* in = a == 0 ? iu : (a == 1 ? iv : iw);
         const T* sup = a == 0 ? su : (a == 1 ? sv : sw);
-        int fi = int(f % g.fc[a][0]);
-        int fj = int((f / g.fc[a][0]) % g.fc[a][1]);
-        int fk = int(f / ((long long)g.fc[a][0] * g.fc[a][1]));
+        int fi, fj, fk;
+        face_coords(g, a, int(f), fi, fj, fk);
         T expect = in[f];
         if (!is_wall_face(g, a, fi, fj, fk)) {
             const int c = cell_idx(g, fi, fj, fk);
@@ -287,8 +306,10 @@ int launch_projection_witness(const GridDev& g, const double* p, double dt, cons
                                      int*, cudaStream_t);                                           \
     template int launch_divergence<T>(const GridDev&, const T*, const T*, const T*, double*, int*,  \
                                       cudaStream_t);                                                \
-    template int launch_correct<T>(const GridDev&, const double*, double, T*, T*, T*, int*,         \
-                                   cudaStream_t);                                                   \
+    template int launch_build_rhs_checked<T>(const GridDev&, const T*, const T*, const T*, double,  \
+                                             double*, int*, cudaStream_t);                          \
+    template int launch_correct<T>(const GridDev&, const double*, double, T*, T*, T*, const int*,   \
+                                   int*, cudaStream_t);                                             \
     template int launch_correct_divergence<T>(const GridDev&, const double*, double,                \
                                               const T* const[3], T* const[3], Partials, int,        \
                                               double*, int*, cudaStream_t);                         \

@@ -17,23 +17,50 @@ constexpr float kF32Max = 3.40282346638528859811704183484516925440e+38f;
 // RN(1/x) where div_diag may use it (2^-500 < x < 2^500), else 0.
 __device__ __forceinline__ double div_reciprocal(double x) { return (x > 0x1p-500 && x < 0x1p500) ? 1.0 / x : 0.0; }
 
-template <class T>
+// The flags of a cell's lower faces and, at the end of an axis, its upper wall.
+__device__ __forceinline__ int face_checks(const GridDev& g, int i, int j, int k, const double lo[3],
+                                           const double hi[3]) {
+    const int p[3] = {i, j, k};
+    int f = 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        if (!isfinite(lo[a])) f |= VF_NONFINITE;
+        if (p[a] == 0 && lo[a] != 0.0) f |= VF_WALL;
+        if (p[a] + 1 == g.n[a]) {
+            if (!isfinite(hi[a])) f |= VF_NONFINITE;
+            if (hi[a] != 0.0) f |= VF_WALL;
+        }
+    }
+    return f;
+}
+
+// CHECK: validate_velocity (src/operator.rs:850-875) on the way, every face by
+// the cell it is the lower face of (the upper walls by the last cells): finite,
+// wall-normal faces zero.
+template <class T, bool CHECK = false>
 __device__ __forceinline__ void build_rhs_body(const GridDev& g, const T* __restrict__ u, const T* __restrict__ v,
                                                const T* __restrict__ w, double dt, double* __restrict__ out,
                                                int* flags, Span sp) {
     // flux / dt correctly rounded through RN(1/dt) and one exact remainder
     const double rdt = div_reciprocal(dt);
+    int local = 0;
     for (int c = sp.block * blockDim.x + threadIdx.x; c < g.cells; c += sp.blocks * blockDim.x) {
         int i, j, k;
         cell_coords(g, c, i, j, k);
+        const double lo[3] = {double(u[face_idx(g, 0, i, j, k)]), double(v[face_idx(g, 1, i, j, k)]),
+                              double(w[face_idx(g, 2, i, j, k)])};
+        const double hi[3] = {double(u[face_idx(g, 0, i + 1, j, k)]), double(v[face_idx(g, 1, i, j + 1, k)]),
+                              double(w[face_idx(g, 2, i, j, k + 1)])};
+        if (CHECK) local |= face_checks(g, i, j, k, lo, hi);
         double flux = 0.0;
-        flux += g.area[0] * (double(u[face_idx(g, 0, i, j, k)]) - double(u[face_idx(g, 0, i + 1, j, k)]));
-        flux += g.area[1] * (double(v[face_idx(g, 1, i, j, k)]) - double(v[face_idx(g, 1, i, j + 1, k)]));
-        flux += g.area[2] * (double(w[face_idx(g, 2, i, j, k)]) - double(w[face_idx(g, 2, i, j, k + 1)]));
+        flux += g.area[0] * (lo[0] - hi[0]);
+        flux += g.area[1] * (lo[1] - hi[1]);
+        flux += g.area[2] * (lo[2] - hi[2]);
         double value = div_diag(flux, dt, rdt);
-        if (!isfinite(value)) atomicOr(flags, VF_ARITH);
+        if (!isfinite(value)) local |= VF_ARITH;
         out[c] = value;
     }
+    if (local) atomicOr(flags, local);
 }
 
 // ------------------------------------------------------------ divergence
