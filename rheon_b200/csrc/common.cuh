@@ -160,6 +160,22 @@ __device__ __forceinline__ dd dd_shfl_xor(dd a, int m) {
     return r;
 }
 
+// Sum of two compensated pairs without renormalising (the value is hi + lo):
+// half the dependent operations of dd_add, which a reduction tree is made of.
+__device__ __forceinline__ dd pair_add(dd a, dd b) {
+    dd r;
+    double e;
+    two_sum(a.hi, b.hi, r.hi, e);
+    r.lo = (a.lo + b.lo) + e;
+    return r;
+}
+template <int LANES>
+__device__ __forceinline__ dd lanes_sum(dd a) {
+#pragma unroll
+    for (int m = LANES / 2; m >= 1; m >>= 1) a = pair_add(a, dd_shfl_xor(a, m));
+    return a;
+}
+
 __device__ __forceinline__ dd warp_reduce_dd(dd a) {
 #pragma unroll
     for (int m = 16; m >= 1; m >>= 1) a = dd_add(a, dd_shfl_xor(a, m));

@@ -20,6 +20,7 @@
 #include <cfloat>
 
 #include "liquid.hpp"
+#include "slab.cuh"
 
 namespace rb200 {
 namespace {
@@ -296,7 +297,31 @@ __device__ __forceinline__ void block_max(double (&m)[LQ_M], double (*sm)[LQ_M])
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(LQ_THREADS) k_liquid_advance(LqArgs a) {
+// Block sums into thread 0; without `rare` the boundary and source sums (2..5)
+// are zero everywhere and stay so.
+__device__ __forceinline__ void block_sums(dd (&s)[LQ_K], bool rare, BlockReduce<LQ_K, 0>& sm) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int NW = LQ_THREADS / 32;
+#pragma unroll
+    for (int q = 0; q < LQ_K; ++q)
+        if (rare || q < 2 || q > 5) s[q] = lanes_sum<32>(s[q]);
+    if (lane == 0)
+#pragma unroll
+        for (int q = 0; q < LQ_K; ++q) sm.s[warp][q] = s[q];
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+        for (int q = 0; q < LQ_K; ++q)
+            if (rare || q < 2 || q > 5) s[q] = lanes_sum<NW>(sm.s[lane & (NW - 1)][q]);
+    }
+    __syncthreads();
+}
+
+// Bound by issue (about 800 instructions a cell, the products' checks most of
+// them) with 126 registers a thread; two blocks per SM for the whole launch, so
+// that the 20-value block reduction runs once per resident block and the last
+// block folds 296 partials instead of 1184: 82 us for 150x96x75, 131 before.
+__global__ void __launch_bounds__(LQ_THREADS, 2) k_liquid_advance(LqArgs a) {
     __shared__ BlockReduce<LQ_K, 0> red;
     __shared__ double smax[32][LQ_M];
     __shared__ bool last;
@@ -318,22 +343,18 @@ __global__ void __launch_bounds__(LQ_THREADS) k_liquid_advance(LqArgs a) {
     v.periodic = f.periodic;
     for (int d = 0; d < 3; ++d) v.rh[d] = a.L->rh[d];
     v.rvol = a.L->rvolume;
-    dd sums[LQ_K];
+    // compensated per-thread sums; the boundary and source terms (`rare`) are
+    // reduced only where a block has any
+    Neu vol[2], rare[4];
     double maxs[LQ_M] = {0.0, 0.0, -INFINITY, -INFINITY};
-#pragma unroll
-    for (int q = 0; q < LQ_K; ++q) sums[q] = dd{0.0, 0.0};
+    bool has_rare = v.src != nullptr;
     bool face_bad = false, vel_bad = false, src_bad = false;
     unsigned dry = 0u, full = 0u;
     const int n0 = g.n[0], n01 = g.n[0] * g.n[1];
-    // one warp per row (j, k) of cells, lanes along x: coalesced accesses and
-    // one division per row instead of two per cell
-    const int rows = g.n[1] * g.n[2];
     const int lane = threadIdx.x & 31;
-    const int warps = gridDim.x * (LQ_THREADS / 32);
-    for (int row = blockIdx.x * (LQ_THREADS / 32) + (threadIdx.x >> 5); row < rows; row += warps)
-    for (int i = lane; i < n0; i += 32) {
-        const int k = row / g.n[1], j = row - k * g.n[1];
-        const int c = i + n0 * row;
+    for (int c = blockIdx.x * LQ_THREADS + threadIdx.x; c < g.cells; c += gridDim.x * LQ_THREADS) {
+        int i, j, k;
+        cell_coords(g, c, i, j, k);
         if (v.periodic) {
             // seams (src/liquid_volume.rs:530-554): a lower boundary face and
             // its upper partner carry the same velocity
@@ -354,15 +375,16 @@ __global__ void __launch_bounds__(LQ_THREADS) k_liquid_advance(LqArgs a) {
             continue;
         }
         v.cand[c] = o.fraction;
-        sums[0] = dd_add1(sums[0], v.volume * v.acc[c]);
-        sums[1] = dd_add1(sums[1], v.volume * o.fraction);
+        vol[0].add(v.volume * v.acc[c]);
+        vol[1].add(v.volume * o.fraction);
         if (i == 0 || j == 0 || k == 0 || i + 1 == g.n[0] || j + 1 == g.n[1] || k + 1 == g.n[2]) {
-            sums[2] = dd_add1(sums[2], o.inward);
-            sums[3] = dd_add1(sums[3], o.outward);
+            has_rare = true;
+            rare[0].add(o.inward);
+            rare[1].add(o.outward);
         }
         if (v.src) {
-            sums[4] = dd_add1(sums[4], o.source);
-            sums[5] = dd_add1(sums[5], fabs(o.source));
+            rare[2].add(o.source);
+            rare[3].add(fabs(o.source));
         }
         dry += o.fraction == 0.0 ? 1u : 0u;
         full += o.fraction == 1.0 ? 1u : 0u;
@@ -374,12 +396,17 @@ __global__ void __launch_bounds__(LQ_THREADS) k_liquid_advance(LqArgs a) {
     if (__syncthreads_or(face_bad) && threadIdx.x == 0) atomicOr(&a.sc.flags[0], 1);
     if (__syncthreads_or(vel_bad) && threadIdx.x == 0) atomicOr(&a.sc.flags[1], 1);
     if (__syncthreads_or(src_bad) && threadIdx.x == 0) atomicOr(&a.sc.flags[2], 1);
+    dd sums[LQ_K];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) sums[q] = dd{vol[q].s, vol[q].c};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) sums[2 + q] = dd{rare[q].s, rare[q].c};
     // occupancy counts (exact in a double: fewer than 2^53 cells)
-    sums[6] = dd{double(__reduce_add_sync(0xffffffffu, dry)), 0.0};
-    sums[7] = dd{double(__reduce_add_sync(0xffffffffu, full)), 0.0};
-    if ((threadIdx.x & 31) != 0) sums[6] = sums[7] = dd{0.0, 0.0};
-    double none[1] = {0.0};
-    block_reduce<LQ_K, 0>(red, sums, none);
+    dry = __reduce_add_sync(0xffffffffu, dry);
+    full = __reduce_add_sync(0xffffffffu, full);
+    sums[6] = dd{lane == 0 ? double(dry) : 0.0, 0.0};
+    sums[7] = dd{lane == 0 ? double(full) : 0.0, 0.0};
+    block_sums(sums, __syncthreads_or(has_rare) != 0, red);
     block_max(maxs, smax);
     if (threadIdx.x == 0) {
         double* slot = a.sc.part + size_t(blockIdx.x) * LQ_STRIDE;
@@ -404,11 +431,11 @@ __global__ void __launch_bounds__(LQ_THREADS) k_liquid_advance(LqArgs a) {
     for (int b = threadIdx.x; b < int(gridDim.x); b += LQ_THREADS) {
         const double* slot = a.sc.part + size_t(b) * LQ_STRIDE;
 #pragma unroll
-        for (int q = 0; q < LQ_K; ++q) sums[q] = dd_add(sums[q], dd{__ldcg(slot + 2 * q), __ldcg(slot + 2 * q + 1)});
+        for (int q = 0; q < LQ_K; ++q) sums[q] = pair_add(sums[q], dd{__ldcg(slot + 2 * q), __ldcg(slot + 2 * q + 1)});
 #pragma unroll
         for (int q = 0; q < LQ_M; ++q) maxs[q] = fmax(maxs[q], __ldcg(slot + 2 * LQ_K + q));
     }
-    block_reduce<LQ_K, 0>(red, sums, none);
+    block_sums(sums, true, red);
     block_max(maxs, smax);
     if (threadIdx.x == 0) {
         int flags[3];
@@ -487,7 +514,7 @@ bool host_product(double a, double b, double* out) {
 }  // namespace
 
 int liquid_blocks(const GridDev& g) {
-    return std::max(1, std::min((g.cells + LQ_THREADS - 1) / LQ_THREADS, 148 * 8));
+    return std::max(1, std::min((g.cells + LQ_THREADS - 1) / LQ_THREADS, 148 * 2));
 }
 
 size_t liquid_partial_doubles(int blocks) { return size_t(blocks) * LQ_STRIDE; }

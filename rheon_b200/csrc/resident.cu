@@ -95,22 +95,6 @@ __device__ __forceinline__ double row_at(const GridDev& g, double cv, double xm,
     return q;
 }
 
-// Sum of two compensated pairs without renormalising (the value is hi + lo):
-// half the dependent operations of dd_add, which a reduction tree is made of.
-__device__ __forceinline__ dd pair_add(dd a, dd b) {
-    dd r;
-    double e;
-    two_sum(a.hi, b.hi, r.hi, e);
-    r.lo = (a.lo + b.lo) + e;
-    return r;
-}
-template <int LANES>
-__device__ __forceinline__ dd lanes_sum(dd a) {
-#pragma unroll
-    for (int m = LANES / 2; m >= 1; m >>= 1) a = pair_add(a, dd_shfl_xor(a, m));
-    return a;
-}
-
 struct Neu2 {
     Neu a, b;
     __device__ __forceinline__ dd as_dd() const { return pair_add(dd{a.s, a.c}, dd{b.s, b.c}); }
