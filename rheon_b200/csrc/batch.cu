@@ -453,7 +453,7 @@ __global__ void k_b_end_trip_out(BatchInstDev* inst, int count, int max_trips, i
     if (threadIdx.x == 0) *out = any;
 }
 
-__global__ void __launch_bounds__(BT) k_b_correct(const BatchInstDev* __restrict__ inst, const __grid_constant__ BatchSpans spans) {
+__global__ void __launch_bounds__(BT, 2) k_b_correct(const BatchInstDev* __restrict__ inst, const __grid_constant__ BatchSpans spans) {
     __shared__ GridDev g;
     Span sp;
     const BatchInstDev& I = inst[batch_entry(spans, sp)];

@@ -20,7 +20,7 @@ __global__ void __launch_bounds__(DCT_THREADS, 2) k_dct(const __grid_constant__ 
     dct_tile_any<ROW, OP>(J, blockIdx.x, cold, reinterpret_cast<float*>(dct_smem));
 }
 
-__global__ void __launch_bounds__(MG_THREADS) k_refine(GridDev g, SolveState* st, const double* b, double* pa,
+__global__ void __launch_bounds__(MG_THREADS, 3) k_refine(GridDev g, SolveState* st, const double* b, double* pa,
                                                        double* pb, const float* z, float* r32, Partials part,
                                                        rb200_trace* trace, int seed, int kc_len) {
     pdl_wait();
@@ -30,8 +30,11 @@ __global__ void __launch_bounds__(MG_THREADS) k_refine(GridDev g, SolveState* st
 __global__ void __launch_bounds__(256) k_settle(int cells, const SolveState* st, double* __restrict__ pa,
                                                 const double* __restrict__ pb) {
     pdl_wait();
-    if (!(st->flags & F_DONE) || !st->dsel) return;
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < cells; c += gridDim.x * blockDim.x) pa[c] = pb[c];
+    if (!(st->flags & F_DONE)) return;
+    const bool zero = settle_zero(st);
+    if (!zero && !st->dsel) return;
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < cells; c += gridDim.x * blockDim.x)
+        pa[c] = zero ? 0.0 : pb[c];
 }
 
 // ------------------------------------------------------------ host side
