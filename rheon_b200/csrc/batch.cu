@@ -289,6 +289,21 @@ __global__ void __launch_bounds__(DCT_THREADS, 2) k_b_dct(const BatchDctJob* __r
     dct_tile_any<ROW, OP>(J, sp.block, J.src64 != nullptr && st->it == 0, reinterpret_cast<float*>(dct_smem));
 }
 
+// The right-hand side and the solve's start of the direct instances.
+__global__ void __launch_bounds__(BT) k_b_rhs_init(const BatchInstDev* __restrict__ inst,
+                                                   const BatchRefine* __restrict__ ref,
+                                                   const __grid_constant__ BatchSpans spans) {
+    __shared__ GridDev g;
+    Span sp;
+    const BatchInstDev& I = inst[ref[batch_entry(spans, sp)].inst];
+    load_geometry(g, I.g);
+    __syncthreads();
+    BatchStepDev* cd = I.step;
+    if (!running(cd)) return;
+    const int b = (cd->acc + 1) % 3;
+    rhs_init_body<float>(g, I.faces[b][0], I.faces[b][1], I.faces[b][2], cd->dt, I.b, &cd->flags, I.st, I.part, sp);
+}
+
 __global__ void __launch_bounds__(MG_THREADS) k_b_refine(const BatchInstDev* __restrict__ inst,
                                                          const BatchRefine* __restrict__ ref,
                                                          const __grid_constant__ BatchSpans spans, int kc_len) {
@@ -309,8 +324,10 @@ __global__ void __launch_bounds__(BT) k_b_settle(const BatchInstDev* __restrict_
     pdl_wait();
     Span sp;
     const BatchInstDev& I = inst[ref[batch_entry(spans, sp)].inst];
-    if (!(I.st->flags & F_DONE) || !I.st->dsel) return;
-    for (int c = sp.block * BT + threadIdx.x; c < I.g.cells; c += sp.blocks * BT) I.p[c] = I.d0[c];
+    if (!(I.st->flags & F_DONE)) return;
+    const bool zero = settle_zero(I.st);
+    if (!zero && !I.st->dsel) return;
+    for (int c = sp.block * BT + threadIdx.x; c < I.g.cells; c += sp.blocks * BT) I.p[c] = zero ? 0.0 : I.d0[c];
 }
 
 // ------------------------------------------------------------ flexible-CG passes
@@ -890,7 +907,7 @@ struct Emit {
             }
         }
     }
-    // dt policy, advection, RHS (then the solve's timing event in a graph)
+    // dt policy, advection (then the solve's timing event in a graph)
     void head() {
         const int ib = ceil_div(B->count, 128);
         go(KK_BEGIN, false, k_b_begin, ib, 128, 0, B->inst_d, B->count);
@@ -898,14 +915,19 @@ struct Emit {
             go(KK_ADVECT, false, k_b_advect<float>, total_blocks(B->sp_faces), BT, 0, B->inst_d, B->sp_faces);
         else
             go(KK_ADVECT, false, k_b_advect<double>, total_blocks(B->sp_faces), BT, 0, B->inst_d, B->sp_faces);
-        go(KK_RHS, false, k_b_rhs, total_blocks(B->sp_cells), BT, 0, B->inst_d, B->sp_cells);
     }
-    // the solve's start: state, compatibility sums; for the multigrid
-    // instances the residual and first V-cycle
+    // the solve's start: state, right-hand side and compatibility sums (one
+    // pass for the direct instances); for the multigrid instances the residual
+    // and first V-cycle
     void start() {
         const int ib = ceil_div(B->count, 128);
         go(KK_RESET, false, k_b_reset, ib, 128, 0, B->inst_d, B->count, B->cfg.settings);
-        go(KK_SUMS, false, k_b_init_sums, total_blocks(B->sp_cells), BT, 0, B->inst_d, B->sp_cells);
+        if (B->direct_count)
+            go(KK_RHS, false, k_b_rhs_init, total_blocks(B->sp_settle), BT, 0, B->inst_d,
+               static_cast<const BatchRefine*>(B->refine_d), B->sp_settle);
+        if (!B->mg_count) return;
+        go(KK_RHS, false, k_b_rhs, total_blocks(B->sp_cells_mg), BT, 0, B->inst_d, B->sp_cells_mg);
+        go(KK_SUMS, false, k_b_init_sums, total_blocks(B->sp_cells_mg), BT, 0, B->inst_d, B->sp_cells_mg);
     }
     void mg_start() {
         go(KK_LOAD, false, k_b_load_residual, total_blocks(B->sp_cells_mg), BT, 0, B->inst_d, B->sp_cells_mg,

@@ -18,6 +18,7 @@
 #include "advect.cuh"
 #include "internal.hpp"
 #include "carrier.hpp"
+#include "direct_device.cuh"
 #include "project.cuh"
 
 namespace rb200 {
@@ -73,6 +74,16 @@ __global__ void k_carrier_rhs(GridDev g, CarrierDev* cd, double* __restrict__ rh
     const int b = (cd->acc + 1) % 3;
     build_rhs_body<T>(g, (const T*)cd->faces[b][0], (const T*)cd->faces[b][1], (const T*)cd->faces[b][2], cd->dt,
                       rhs, &cd->flags, whole_launch());
+}
+
+// The right-hand side and the start of a cold direct solve.
+template <class T>
+__global__ void __launch_bounds__(EW_THREADS) k_carrier_rhs_init(GridDev g, CarrierDev* cd, double* __restrict__ rhs,
+                                                                 SolveState* st, Partials part) {
+    if (!step_running(cd)) return;
+    const int b = (cd->acc + 1) % 3;
+    rhs_init_body<T>(g, (const T*)cd->faces[b][0], (const T*)cd->faces[b][1], (const T*)cd->faces[b][2], cd->dt, rhs,
+                     &cd->flags, st, part, whole_launch());
 }
 
 template <class T>
@@ -282,9 +293,16 @@ int capture_step(rb200_carrier* c) {
         k_carrier_advect<T, float><<<fb, ADV_THREADS, 0, s>>>(g, c->cd);
     else
         k_carrier_advect<T, double><<<fb, ADV_THREADS, 0, s>>>(g, c->cd);
-    k_carrier_rhs<T><<<cb, ADV_THREADS, 0, s>>>(g, c->cd, c->solver.b());
+    int rc = RB200_OK;
+    const bool fused = !c->accepted_p && c->solver.fuses_rhs();
+    if (!fused) k_carrier_rhs<T><<<cb, ADV_THREADS, 0, s>>>(g, c->cd, c->solver.b());
     RB200_CUDA(cudaEventRecordWithFlags(c->ev[0], s, cudaEventRecordExternal));
-    int rc = c->accepted_p
+    if (fused) {
+        rc = c->solver.enqueue_reset_fused(&c->cd->dt, &c->cd->skip, c->cfg.settings, s);
+        k_carrier_rhs_init<T><<<eb, EW_THREADS, 0, s>>>(g, c->cd, c->solver.b(), c->solver.state(),
+                                                        c->solver.partials());
+    } else
+        rc = c->accepted_p
                  ? c->solver.enqueue_reset(&c->cd->dt, &c->cd->skip, c->cfg.settings, s, &c->cd->warm, c->accepted_p)
                  : c->solver.enqueue_reset(&c->cd->dt, &c->cd->skip, c->cfg.settings, s);
     if (!rc) rc = c->solver.enqueue_loop(s, c->body_stream, c->cfg.settings);

@@ -99,7 +99,8 @@ public:
     // state's dsel tells which holds it). Returns the number of launches.
     int enqueue_iteration(const GridDev& g, SolveState* st, const double* b, double* p, double* p2, Partials part,
                           rb200_trace* trace, cudaStream_t s) const;
-    // Copies a finished iterate from p2 to p where it ended there.
+    // Copies a finished iterate from p2 to p where it ended there; p = 0 where
+    // the solve ended before its first iteration.
     int enqueue_settle(const GridDev& g, SolveState* st, double* p, const double* p2, cudaStream_t s) const;
     size_t bytes() const { return bytes_; }
 

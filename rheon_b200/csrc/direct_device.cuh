@@ -5,6 +5,8 @@
 
 #include "direct.hpp"
 #include "mg_device.cuh"
+#include "pcg_device.cuh"
+#include "project.cuh"
 
 namespace rb200 {
 
@@ -372,6 +374,94 @@ __device__ __forceinline__ void dct_tile_any(const DctJob& J, int tile, bool col
         dct_tile<6, ROW, OP>(J, tile, cold, smem);
     else
         dct_tile<4, ROW, OP>(J, tile, cold, smem);
+}
+
+// build_rhs (project.cuh) with the start of a cold solve on it (the sums of b,
+// |b| and b^2, max|b| and the decision of init_sums_body, pcg_device.cuh) in
+// one pass: b is written once and not read back, and p is not zeroed (a solve
+// that ends at iteration 0 has it zeroed by k_settle). Rows of a multiple of 4
+// cells take quads and march along z as correct_divergence_quads does. Bound by
+// HBM (20 bytes a cell in f32). The two passes it replaces took 101 + 97 us at
+// 256^3 on a B200 and 0.28 + 0.25 ms over 64 boxes of 32^3 to 96^3; this one
+// about 100 us and 0.26 ms.
+template <class T>
+__device__ __forceinline__ void rhs_init_body(const GridDev& g, const T* __restrict__ u, const T* __restrict__ v,
+                                              const T* __restrict__ w, double dt, double* __restrict__ out, int* vflags,
+                                              SolveState* st, Partials part, Span sp) {
+    __shared__ BlockReduce<3, 3> sm;
+    const double rdt = div_reciprocal(dt);
+    const int n0 = g.n[0], n1 = g.n[1], n2 = g.n[2];
+    Neu sum[3];
+    double m[3] = {0.0, 0.0, 0.0};
+    int local = 0;
+    auto value = [&](T xl, T xh, T yl, T yh, T zl, T zh) {
+        double flux = 0.0;
+        flux += g.area[0] * (double(xl) - double(xh));
+        flux += g.area[1] * (double(yl) - double(yh));
+        flux += g.area[2] * (double(zl) - double(zh));
+        const double b = div_diag(flux, dt, rdt);
+        if (!isfinite(b)) {
+            local |= VF_ARITH;
+            m[1] = 1.0;
+        }
+        const double a = fabs(b);
+        sum[0].add(b);
+        sum[1].add(a);
+        sum[2].add(b * b);
+        m[0] = a > m[0] ? a : m[0];
+        return b;
+    };
+    if ((n0 & 3) == 0) {
+        const int quads = n0 >> 2, sz = n0 * n1;
+        const int items = quads * n1, segs = (items + 31) >> 5;
+        const int lane = threadIdx.x & 31, nw = sp.blocks * int(blockDim.x >> 5);
+        const int kc = march_planes(segs, n2, nw), kcs = (n2 + kc - 1) / kc;
+        for (int line = sp.block * int(blockDim.x >> 5) + int(threadIdx.x >> 5); line < segs * kcs; line += nw) {
+            const int seg = line % segs, kb = (line / segs) * kc, ke = min(n2, kb + kc);
+            const int it = seg * 32 + lane;
+            if (it >= items) continue;
+            const int j = it / quads, i0 = 4 * (it - j * quads);
+            int c = i0 + n0 * (j + n1 * kb);
+            T wl[4];
+            ld4(w + c, wl);
+            for (int k = kb; k < ke; ++k, c += sz) {
+                const int fu = i0 + (n0 + 1) * (j + n1 * k), fv = i0 + n0 * (j + (n1 + 1) * k);
+                T x[5], vl[4], vh[4], wh[4];
+#pragma unroll
+                for (int e = 0; e < 5; ++e) x[e] = u[fu + e];
+                ld4(v + fv, vl);
+                ld4(v + fv + n0, vh);
+                ld4(w + c + sz, wh);
+                double b[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    b[e] = value(x[e], x[e + 1], vl[e], vh[e], wl[e], wh[e]);
+                    wl[e] = wh[e];
+                }
+                st4(out + c, b);
+            }
+        }
+    } else {
+        for (int c = sp.block * blockDim.x + threadIdx.x; c < g.cells; c += sp.blocks * blockDim.x) {
+            int i, j, k;
+            cell_coords(g, c, i, j, k);
+            out[c] = value(u[face_idx(g, 0, i, j, k)], u[face_idx(g, 0, i + 1, j, k)], v[face_idx(g, 1, i, j, k)],
+                           v[face_idx(g, 1, i, j + 1, k)], w[face_idx(g, 2, i, j, k)], w[face_idx(g, 2, i, j, k + 1)]);
+        }
+    }
+    if (local) atomicOr(vflags, local);
+    dd s[3] = {sum[0].as_dd(), sum[1].as_dd(), sum[2].as_dd()};
+    block_reduce<3, 3>(sm, s, m);
+    if (publish_and_check_last<3, 3>(part, sp.block, sp.blocks, s, m)) {
+        fold_partials<3, 3>(part, sp.blocks, sm, s, m);
+        if (threadIdx.x == 0) decide_init(g, st, s, m, false, nullptr);
+    }
+}
+
+// Whether a finished solve left p untouched: it ended on the right-hand side,
+// and p = 0 is its result.
+__device__ __forceinline__ bool settle_zero(const SolveState* st) {
+    return st->it == 0 && !(st->flags & F_WARM) && st->status != ST_RUNNING;
 }
 
 // Decision after a refinement iteration's true residual (`squared`, `maximum`

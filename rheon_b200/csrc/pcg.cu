@@ -1240,6 +1240,15 @@ int PcgSolver::enqueue_reset(const double* dt_dev, const int* skip, const rb200_
     return RB200_OK;
 }
 
+int PcgSolver::enqueue_reset_fused(const double* dt_dev, const int* skip, const rb200_settings& settings,
+                                   cudaStream_t s) {
+    k_solve_reset<<<1, 1, 0, s>>>(st_, settings, dt_dev, skip, 1, nullptr);
+    RB200_CUDA(cudaMemsetAsync(part_.ticket, 0, sizeof(unsigned), s));
+    launches_ += 1;
+    RB200_CUDA(cudaGetLastError());
+    return RB200_OK;
+}
+
 int PcgSolver::enqueue_loop(cudaStream_t cs, cudaStream_t body_stream, const rb200_settings& settings) {
     cudaStreamCaptureStatus status;
     cudaGraph_t graph = nullptr;

@@ -128,6 +128,10 @@ public:
     // g.cells values): the resident carrier's accepted previous pressure.
     int enqueue_reset(const double* dt_dev, const int* skip, const rb200_settings& settings, cudaStream_t s,
                       const int* warm = nullptr, const double* seed = nullptr);
+    // A cold solve by the direct method whose right-hand side is assembled by
+    // rhs_init_body: only the state is reset here, the pass decides the start.
+    bool fuses_rhs() const { return use_direct_; }
+    int enqueue_reset_fused(const double* dt_dev, const int* skip, const rb200_settings& settings, cudaStream_t s);
     int enqueue_loop(cudaStream_t capture_stream, cudaStream_t body_stream, const rb200_settings& settings);
     int nodes_per_chunk() const { return nodes_per_chunk_ + 1; }
     // Blocks of the persistent solver kernel (0: the per-pass kernels run).

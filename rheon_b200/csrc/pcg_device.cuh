@@ -13,6 +13,68 @@ namespace rb200 {
 
 constexpr double kEps = 2.220446049250313e-16;
 
+// The decision of the start (src/pressure.rs:603-650) from the sums of b, |b|
+// and b^2 and the maxima: |b|, a non-finite b, a non-finite seed. Thread 0.
+__device__ __forceinline__ void decide_init(const GridDev& g, SolveState* st, const dd (&s)[3], const double (&m)[3],
+                                            bool warm, const double* p) {
+    int flags = st->flags;
+    if (m[1] != 0.0) {
+        finish(st, RB200_NONFINITE_INPUT, flags);
+        return;
+    }
+    double sum = dd_value(s[0]), sum_abs = dd_value(s[1]), sq = dd_value(s[2]);
+    double budget = (64.0 * kEps) * sum_abs;
+    if (!isfinite(sum) || !isfinite(sum_abs)) {
+        breakdown(st, 0, flags);
+        return;
+    }
+    if (fabs(sum) > budget) {
+        st->incompatible_sum = sum;
+        st->incompatible_budget = budget;
+        finish(st, RB200_INCOMPATIBLE_RHS, flags);
+        return;
+    }
+    if (warm) {
+        if (m[2] != 0.0) {
+            finish(st, RB200_NONFINITE_INPUT, flags);
+            return;
+        }
+        if (p[0] != 0.0) {
+            finish(st, RB200_INVALID_INITIAL_PRESSURE, flags);
+            return;
+        }
+    }
+    double rhs_l2 = sqrt(sq);
+    double threshold = fmax(st->absolute, st->relative * rhs_l2);
+    if (!isfinite(rhs_l2) || !isfinite(threshold)) {
+        breakdown(st, 0, flags);
+        return;
+    }
+    st->threshold = threshold;
+    if (warm) {
+        // true_report(p0) runs next, in the true-residual kernel.
+        st->flags = flags | F_STOP | F_NEED_TRUE;
+        return;
+    }
+    // true_report(p = 0): the product is exactly b.
+    double div = m[0] * st->dt / g.volume;
+    if (!isfinite(sq) || !isfinite(div)) {
+        breakdown(st, 0, flags);
+        return;
+    }
+    st->true_l2 = rhs_l2;
+    st->true_max = m[0];
+    st->true_div = div;
+    if (rhs_l2 <= threshold && div <= st->divergence_limit) {
+        finish(st, RB200_OK, flags);
+        return;
+    }
+    if (st->max_it == 0) {
+        finish(st, RB200_ITERATION_LIMIT, flags);
+        return;
+    }
+}
+
 // ------------------------------------------------------------------ init
 // Compatibility sums, threshold and the true report of p = 0
 // (src/pressure.rs:603-647); p is zeroed here. A seeded solve (F_WARM) keeps p,
@@ -42,64 +104,7 @@ __device__ __forceinline__ void init_sums_body(const GridDev& g, SolveState* st,
     block_reduce<3, 3>(sm, s, m);
     if (publish_and_check_last<3, 3>(part, sp.block, sp.blocks, s, m)) {
         fold_partials<3, 3>(part, sp.blocks, sm, s, m);
-        if (threadIdx.x == 0) {
-            int flags = st->flags;
-            if (m[1] != 0.0) {
-                finish(st, RB200_NONFINITE_INPUT, flags);
-                return;
-            }
-            double sum = dd_value(s[0]), sum_abs = dd_value(s[1]), sq = dd_value(s[2]);
-            double budget = (64.0 * kEps) * sum_abs;
-            if (!isfinite(sum) || !isfinite(sum_abs)) {
-                breakdown(st, 0, flags);
-                return;
-            }
-            if (fabs(sum) > budget) {
-                st->incompatible_sum = sum;
-                st->incompatible_budget = budget;
-                finish(st, RB200_INCOMPATIBLE_RHS, flags);
-                return;
-            }
-            if (warm) {
-                if (m[2] != 0.0) {
-                    finish(st, RB200_NONFINITE_INPUT, flags);
-                    return;
-                }
-                if (p[0] != 0.0) {
-                    finish(st, RB200_INVALID_INITIAL_PRESSURE, flags);
-                    return;
-                }
-            }
-            double rhs_l2 = sqrt(sq);
-            double threshold = fmax(st->absolute, st->relative * rhs_l2);
-            if (!isfinite(rhs_l2) || !isfinite(threshold)) {
-                breakdown(st, 0, flags);
-                return;
-            }
-            st->threshold = threshold;
-            if (warm) {
-                // true_report(p0) runs next, in the true-residual kernel.
-                st->flags = flags | F_STOP | F_NEED_TRUE;
-                return;
-            }
-            // true_report(p = 0): the product is exactly b.
-            double div = m[0] * st->dt / g.volume;
-            if (!isfinite(sq) || !isfinite(div)) {
-                breakdown(st, 0, flags);
-                return;
-            }
-            st->true_l2 = rhs_l2;
-            st->true_max = m[0];
-            st->true_div = div;
-            if (rhs_l2 <= threshold && div <= st->divergence_limit) {
-                finish(st, RB200_OK, flags);
-                return;
-            }
-            if (st->max_it == 0) {
-                finish(st, RB200_ITERATION_LIMIT, flags);
-                return;
-            }
-        }
+        if (threadIdx.x == 0) decide_init(g, st, s, m, warm, p);
     }
 }
 
