@@ -690,9 +690,6 @@ inline size_t train_launch_smem(const MgLevelDev& L, const MgLevelDev& C, int P,
     return train_smem(P, sj, L.n[0], start == TRAIN_PROLONG ? C.n[0] : 0, L.cf[1]);
 }
 
-__device__ __forceinline__ void cp_async16_cg(void* smem_dst, const void* gmem_src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_u32(smem_dst)), "l"(gmem_src) : "memory");
-}
 __device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(smem_u32(smem_dst)), "l"(gmem_src) : "memory");
 }

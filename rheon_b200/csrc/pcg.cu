@@ -353,25 +353,59 @@ __global__ void __launch_bounds__(EW) k_mg_update(GridDev g, SolveState* st, dou
 // (the reference's own tiled wavefront, src/sgs.rs:56-104, uses the same
 // fact).
 //
-// One launch runs both sweeps over 8^3 tiles. A block takes the next slot of
-// a queue (slots 0..T-1: the tiles in wave order tx + ty + tz ascending;
-// T..2T-1: the same list backwards for the reverse sweep), waits until the
-// tiles it depends on are done (forward: the lower x, y, z neighbour tiles;
-// reverse: the upper ones, and for the last tile of the forward order its own
-// forward sweep), stages its tile and the one-cell halo it reads in shared
-// memory, walks the tile's hyperplanes lx + ly + lz = l with a block barrier
-// between them, stores the tile and publishes its state word (release). A
-// slot only waits for slots taken before it, by blocks that are running, so
-// the queue cannot deadlock whatever the number of resident blocks. The
-// reverse sweep of a tile starts after the forward sweep of every tile: its
-// upper neighbours' reverse sweeps come after the forward sweep of the last
-// tile, which comes after every other forward sweep.
+// One launch runs both sweeps over units of 16 x 8 lines along x. A thread
+// owns a line: at step t of a unit, line (j, k) of it does cell i = t - j - k of
+// its direction, so that the x neighbour is the thread's own last value, and the
+// y and z neighbours' are in shared memory since the step before; one barrier a
+// step. What bounds a sweep is that serial chain: n0 + n1 + n2 steps of 160 to
+// 240 cycles (shared load, the sums, each rounded, the division, shared store,
+// barrier), and some 3 us for each unit boundary on the way. So a
+// line's step holds nothing else: a missing neighbour is a -0.0 (adding its
+// product changes no bit), the ends of a line have a path of their own, two
+// warps fetch the next 16 steps' values and store the last 16's through shared
+// memory, 16 consecutive cells of a line at a time, and two warps fetch the
+// unit's incoming faces SGS_AHEAD steps before their use and send the outgoing
+// ones a step after it.
+//
+// A boundary value crosses as two 64-bit words, each a 32-bit half under a tag
+// that holds the sweep's number, which makes a word its own flag. The words lie
+// in the direction buffer that the iteration does not hold (the next pass
+// overwrites it whole); the tags are the bits of signalling NaNs, which no
+// arithmetic leaves there, and both buffers start as zeros.
+//
+// A block takes the next slot of a queue (slots 0..U-1: the units in wave order
+// jb + kb ascending; U..2U-1: the same list backwards for the reverse sweep). A
+// slot only waits for slots taken before it, by blocks that are running, so the
+// queue cannot deadlock whatever the number of resident blocks. A unit's
+// reverse sweep reads the z of its own forward sweep, published by a state word
+// (release); it starts after the forward sweep of every unit, since its upper
+// neighbours' reverse sweeps come after the forward sweep of the last unit,
+// which comes after every other forward sweep.
+//
+// us per iteration of a solve, tiles of 8^3 cells with a block barrier for each
+// of their 22 hyperplanes / this: 32^3 138 / 83, 63x48x37 226 / 108, 96^3
+// 453 / 207, 256x20x20 417 / 124. Units of 16 x 16 lines took 113, 222 and 148
+// for the last three (two line warps to a scheduler), fetching the faces 7
+// steps ahead 120, 238 and 130 (a unit that catches up with its neighbour polls
+// for every word in flight).
 //
 // Every wait is bounded: a wait that runs out raises the abort word, which
 // ends every other wait, and marks the solve as failed (execution error).
-constexpr int SGS_T = 8;
-constexpr int SGS_THREADS = SGS_T * SGS_T * SGS_T;
+constexpr int SGS_UJ = 16, SGS_UK = 8;         // lines of a unit along y and z
+constexpr int SGS_C = 16;                      // steps of a chunk
+constexpr int SGS_P = SGS_C + 1;               // pitch of a line's chunk (bank conflicts)
+constexpr int SGS_LINES = SGS_UJ * SGS_UK;
+constexpr int SGS_MOVERS = 64;                 // threads that move the chunks
+constexpr int SGS_STEPPERS = SGS_LINES + 64;   // the lines and the faces' two warps: they share the step barrier
+constexpr int SGS_THREADS = SGS_STEPPERS + SGS_MOVERS;
+constexpr int SGS_AHEAD = 5;                   // steps between a face word's load and its use
+constexpr int SGS_VP = SGS_UJ + 2;             // pitch of the step values
+constexpr int SGS_VALS = (SGS_UK + 1) * SGS_VP;
+constexpr int SGS_CHUNK = SGS_LINES * SGS_P;
+constexpr int SGS_RING = 8;                    // steps of face words in shared memory
+constexpr size_t kSmemSgs = (3 * SGS_CHUNK + 2 * SGS_VALS + SGS_RING * 64) * sizeof(double);
 constexpr unsigned kSgsSpins = 1u << 22;
+constexpr unsigned kSgsTag = 0x7ff40000u;      // | sweep number mod 2^18
 
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
     unsigned v;
@@ -381,78 +415,353 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
 __device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory");
 }
+__device__ __forceinline__ void ld_pair(const unsigned long long* p, unsigned long long& a, unsigned long long& b) {
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];\n" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void st_tagged(unsigned long long* p, double v, unsigned tag) {
+    const unsigned long long t = (unsigned long long)tag << 32;
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};\n" ::"l"(p), "l"(t | unsigned(__double2loint(v))),
+                 "l"(t | unsigned(__double2hiint(v)))
+                 : "memory");
+}
+// Without a branch: 8 bytes or nothing read (zeros written then); a store or none.
+__device__ __forceinline__ void cp_async8_if(bool on, double* dst, const double* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(smem_u32(dst)), "l"(src), "r"(on ? 8 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void st_cg_if(bool on, double* p, double v) {
+    asm volatile("{\n.reg .pred q;\nsetp.ne.s32 q, %0, 0;\n@q st.global.cg.f64 [%1], %2;\n}\n" ::"r"(int(on)), "l"(p),
+                 "d"(v)
+                 : "memory");
+}
+// Kept out of the step's code, which rarely needs it.
+__device__ __noinline__ double sgs_divide(double a, double b) { return a / b; }
 
-// Wait until tile `dep` holds a state >= need; a wait that runs out raises
-// the abort word.
-__device__ __forceinline__ bool sgs_wait(unsigned* ctl, int dep, unsigned need) {
-    unsigned n = 0;
-    while (ld_acquire_u32(ctl + 2 + dep) < need) {
-        ++n;
-        if ((n & 7u) == 0u && *(volatile const unsigned*)(ctl + 1) != 0u) return false;
-        if (n > kSgsSpins) {
-            atomicExch(ctl + 1, 1u);
-            return false;
-        }
-        if (n > 256u) __nanosleep(64);
-    }
-    return true;
+// The steppers' barrier; at the end of a chunk the whole block's.
+__device__ __forceinline__ void sgs_step_barrier() {
+    asm volatile("bar.sync 1, %0;\n" ::"n"(SGS_STEPPERS) : "memory");
+}
+__device__ __forceinline__ void sgs_step_end(int t, int steps) {
+    if (t + 1 == steps || t % SGS_C == SGS_C - 1)
+        __syncthreads();
+    else
+        sgs_step_barrier();
 }
 
-__global__ void __launch_bounds__(SGS_THREADS) k_sgs_flow(GridDev g, SolveState* st,
-                                                          const double* __restrict__ r, double* z, SgsFlow f,
-                                                          int mode) {
-    __shared__ double zs[SGS_T + 2][SGS_T + 2][SGS_T + 2];  // the tile at [1..8], its halo at 0 and 9
-    __shared__ int s_slot, s_ok;
+// A unit: its place among the units, its first line and its lines.
+struct SgsUnit {
+    int jb, kb, nj, nk, j0, k0;
+};
+// The incoming face words of line `line` of axis y or z (face f lies between
+// units f and f + 1 of that axis).
+__device__ __forceinline__ size_t sgs_word(const GridDev& g, const SgsFlow& f, bool z, int face, int line) {
+    const size_t row = z ? size_t(f.nj - 1) * g.n[2] + size_t(face) * g.n[1] + line
+                         : size_t(face) * g.n[2] + line;
+    return 2 * row * g.n[0];
+}
+
+// Polls a face word until it holds the tag; all lanes of a warp. False when the
+// wait ran out or another did.
+__device__ __noinline__ bool sgs_poll(const unsigned long long* p, unsigned tag, bool want, unsigned* ctl,
+                                      unsigned long long* lo, unsigned long long* hi) {
+    for (unsigned n = 1;; ++n) {
+        unsigned long long a = 0, b = 0;
+        if (want) ld_pair(p, a, b);
+        if (__all_sync(0xffffffffu, !want || (unsigned(a >> 32) == tag && unsigned(b >> 32) == tag))) {
+            *lo = a;
+            *hi = b;
+            return true;
+        }
+        const bool out = n > kSgsSpins || ((n & 7u) == 0u && *(volatile const unsigned*)(ctl + 1) != 0u);
+        if (__any_sync(0xffffffffu, out)) return false;
+    }
+}
+
+// The incoming faces' warp of a unit: lane q fetches line q of the y face, lane
+// 16 + q of the z face, one step of the unit at a time. The words come through
+// asynchronous copies, since a load into registers would be waited for at the
+// next branch; a word that came too early is polled for.
+template <bool REV>
+__device__ __forceinline__ void sgs_faces(const GridDev& g, const SgsFlow& f, const SgsUnit& U, int steps,
+                                          const unsigned long long* words, unsigned tag, double* vals,
+                                          unsigned long long* ring, int* s_fail) {
+    const int lane = threadIdx.x & 31, q = lane & 15, n0 = g.n[0];
+    const bool zf = lane >= 16;
+    const int b = zf ? U.kb : U.jb, nb = zf ? f.nk : f.nj, lines = zf ? U.nj : U.nk;
+    const bool has = q < lines && (REV ? b + 1 < nb : b > 0);
+    const int line = (zf ? U.j0 : U.k0) + (REV ? lines - 1 - q : q);
+    const unsigned long long* base = words + (has ? sgs_word(g, f, zf, REV ? b : b - 1, line) : 0);
+    double* const to = vals + (zf ? q + 1 : (q + 1) * SGS_VP);
+    if (!has) to[0] = to[SGS_VALS] = -0.0;
+    if (!__any_sync(0xffffffffu, has)) {
+        __syncthreads();
+        for (int t = 0; t < steps; ++t) sgs_step_end(t, steps);
+        return;
+    }
+    const unsigned len = has ? unsigned(n0) : 0u;
+    auto wanted = [&](int t) { return unsigned(t - q) < len; };
+    auto word = [&](int t) { return base + 2 * (REV ? n0 - 1 - (t - q) : t - q); };
+    auto fetch = [&](int t) {
+        if (wanted(t)) cp_async16_cg(ring + (t % SGS_RING) * 64 + 2 * lane, word(t));
+        cp_async_commit();
+    };
+    unsigned long long lo, hi;  // the word pair of the next step
+    auto read = [&](int t) {
+        lo = ring[(t % SGS_RING) * 64 + 2 * lane];
+        hi = ring[(t % SGS_RING) * 64 + 2 * lane + 1];
+    };
+    bool dead = false;
+    auto deliver = [&](int t) {
+        const bool want = wanted(t);
+        const bool ok = !want || (unsigned(lo >> 32) == tag && unsigned(hi >> 32) == tag);
+        if (!__all_sync(0xffffffffu, ok) && !dead && !sgs_poll(want ? word(t) : words, tag, want, f.ctl, &lo, &hi)) {
+            dead = true;
+            if (lane == 0) {
+                atomicExch(f.ctl + 1, 1u);
+                *s_fail = 1;
+            }
+        }
+        if (want) to[((t + 1) & 1) * SGS_VALS] = __hiloint2double(int(unsigned(hi)), int(unsigned(lo)));
+    };
+    for (int t = 0; t < SGS_AHEAD; ++t) fetch(t);
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(SGS_AHEAD - 2) : "memory");
+    read(0);
+    deliver(0);
+    read(1);
+    __syncthreads();
+    for (int t = 0; t < steps; ++t) {
+        deliver(t + 1);
+        fetch(t + SGS_AHEAD);
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(SGS_AHEAD - 2) : "memory");
+        read(t + 2);
+        sgs_step_end(t, steps);
+    }
+    cp_async_wait_all();
+}
+
+// The outgoing faces' warp of a unit, one step behind the lines: lane q sends
+// line q of the y face, lane 16 + q of the z face.
+template <bool REV>
+__device__ __forceinline__ void sgs_send(const GridDev& g, const SgsFlow& f, const SgsUnit& U, int steps,
+                                         unsigned long long* words, unsigned tag, const double* vals) {
+    const int lane = threadIdx.x & 31, q = lane & 15, n0 = g.n[0];
+    const bool zf = lane >= 16;
+    const int b = zf ? U.kb : U.jb, nb = zf ? f.nk : f.nj, lines = zf ? U.nj : U.nk;
+    const bool has = q < lines && (REV ? b > 0 : b + 1 < nb);
+    const int line = (zf ? U.j0 : U.k0) + (REV ? lines - 1 - q : q);
+    unsigned long long* const base = words + (has ? sgs_word(g, f, zf, REV ? b - 1 : b, line) : 0);
+    const double* const from = vals + (zf ? U.nk * SGS_VP + q + 1 : (q + 1) * SGS_VP + U.nj);
+    const int back = q + (zf ? U.nk : U.nj) - 1;
+    auto send = [&](int t) {
+        const int i = t - back;
+        if (has && unsigned(i) < unsigned(n0))
+            st_tagged(base + 2 * (REV ? n0 - 1 - i : i), from[(t & 1) * SGS_VALS], tag);
+    };
+    __syncthreads();
+    for (int t = 0; t < steps; ++t) {
+        if (t > 0) send(t - 1);
+        sgs_step_end(t, steps);
+    }
+    send(steps - 1);
+}
+
+// The movers of a unit: chunk c + 1 comes in (r, in reverse z) and chunk c - 1
+// goes out to z while chunk c is computed.
+template <bool REV>
+__device__ __forceinline__ void sgs_move(const GridDev& g, const SgsUnit& U, int steps, const double* __restrict__ r,
+                                         double* z, double* chunks) {
+    constexpr int ROWS = SGS_MOVERS / SGS_C, PASSES = SGS_UJ / ROWS;
+    const int x = threadIdx.x - SGS_STEPPERS, n0 = g.n[0], sz = n0 * g.n[1];
+    const int ts = x % SGS_C, row = x / SGS_C;
+    const double* __restrict__ src = REV ? z : r;
+    // slot ts of line (tj, tk) of a chunk is cell i = 16 chunk + ts - tj - tk of
+    // the line in its direction; from one tk to the next it moves by `hop`
+    const int hop = REV ? 1 - sz : sz - 1;
+    auto start = [&](int chunk, int tj, int& i) {
+        i = chunk * SGS_C + ts - tj;
+        return (REV ? n0 - 1 - i : i) + n0 * (U.j0 + (REV ? U.nj - 1 - tj : tj)) +
+               sz * (U.k0 + (REV ? U.nk - 1 : 0));
+    };
+    auto load = [&](int chunk) {
+        for (int h = 0; h < PASSES; ++h) {
+            const int tj = row + h * ROWS;
+            int i, c = start(chunk, tj, i);
+            double* const dst = chunks + (chunk % 3) * SGS_CHUNK + tj * SGS_P + ts;
+            const unsigned lines = tj < U.nj ? unsigned(U.nk) : 0u;
+#pragma unroll
+            for (int tk = 0; tk < SGS_UK; ++tk) {
+                const bool on = unsigned(tk) < lines && unsigned(i - tk) < unsigned(n0);
+                cp_async8_if(on, dst + tk * SGS_UJ * SGS_P, on ? src + (c + tk * hop) : src);
+            }
+        }
+        cp_async_commit();
+    };
+    auto store = [&](int chunk) {
+        for (int h = 0; h < PASSES; ++h) {
+            const int tj = row + h * ROWS;
+            int i, c = start(chunk, tj, i);
+            const double* const from = chunks + (chunk % 3) * SGS_CHUNK + tj * SGS_P + ts;
+            const unsigned lines = tj < U.nj ? unsigned(U.nk) : 0u;
+            double v[SGS_UK];
+#pragma unroll
+            for (int tk = 0; tk < SGS_UK; ++tk) v[tk] = from[tk * SGS_UJ * SGS_P];
+#pragma unroll
+            for (int tk = 0; tk < SGS_UK; ++tk)
+                st_cg_if(unsigned(tk) < lines && unsigned(i - tk) < unsigned(n0) && c + tk * hop != 0, z + (c + tk * hop), v[tk]);
+        }
+    };
+    const int nchunks = (steps + SGS_C - 1) / SGS_C;
+    load(0);
+    cp_async_wait_all();
+    if (!REV && x == 0 && U.jb == 0 && U.kb == 0) chunks[0] = 0.0;  // the gauge row
+    __syncthreads();
+    for (int ch = 0; ch < nchunks; ++ch) {
+        if (ch + 1 < nchunks) load(ch + 1);
+        if (ch > 0) store(ch - 1);
+        cp_async_wait_all();
+        __syncthreads();
+    }
+    store(nchunks - 1);
+}
+
+// The lines of a unit.
+template <bool REV>
+__device__ __forceinline__ void sgs_lines(const GridDev& g, const SgsUnit& U, int steps, double* chunks,
+                                          double* vals) {
+    const int tid = threadIdx.x, n0 = g.n[0];
+    const int j = tid % SGS_UJ, k = tid / SGS_UJ;
+    const bool line = j < U.nj && k < U.nk;
+    // the divisors at the line's first cell, inside it and at its last cell
+    double D0 = 1.0, y0 = 1.0, D1 = 1.0, y1 = 1.0, Dm = 1.0, ym = 1.0;
+    if (line) {
+        const int jg = U.j0 + (REV ? U.nj - 1 - j : j), kg = U.k0 + (REV ? U.nk - 1 - k : k);
+        const int first = diag_mask(g, REV ? n0 - 1 : 0, jg, kg), end = diag_mask(g, REV ? 0 : n0 - 1, jg, kg);
+        D0 = g.diag[first];
+        y0 = g.rdiag[first];
+        D1 = g.diag[end];
+        y1 = g.rdiag[end];
+        Dm = g.diag[first | 3];
+        ym = g.rdiag[first | 3];
+    }
+    // div_diag_fast_ok on the sum's bits without its sign; no range where a
+    // divisor has no reciprocal (a zero sum is a zero either way)
+    const unsigned range = y0 != 0.0 && y1 != 0.0 && ym != 0.0 ? 901u << 21 : 0u;
+    const double w0 = g.weight[0], w1 = g.weight[1], w2 = g.weight[2];
+    double* const mine = vals + (k + 1) * SGS_VP + j + 1;
+    double last = -0.0;
+    const int back = j + k;
+    // the steps with work for a warp, and the groups of 4 whose cells are all inside
+    const int low = __shfl_sync(0xffffffffu, back, 0), high = __shfl_sync(0xffffffffu, back, 31);
+    const int active = __any_sync(0xffffffffu, line) ? n0 + high - low : 0;
+    const int inside = active ? max(0, n0 - 5 - (high - low)) : 0;
+    auto step = [&](int s, int t, double* cell, bool edge) {
+        const double* const prev = mine + ((s + 1) & 1) * SGS_VALS;
+        const double in = *cell, zy = prev[-1], zz = prev[-SGS_VP];
+        const int i = t - back;
+        const bool on = line && (!edge || unsigned(i) < unsigned(n0));
+        double D = Dm, y = ym;
+        if (edge) {
+            D = i == 0 ? D0 : (i == n0 - 1 ? D1 : Dm);
+            y = i == 0 ? y0 : (i == n0 - 1 ? y1 : ym);
+        }
+        // (r + x + y + z) / D, in reverse y + (0 + x + y + z) / D
+        const double sum = (((REV ? 0.0 : in) + w0 * last) + w1 * zy) + w2 * zz;
+        double v = div_diag_fast(sum, D, y);
+        const unsigned top = unsigned(__double2hiint(sum)) << 1;
+        const bool fast = top - (573u << 21) < range || (top | unsigned(__double2loint(sum))) == 0u;
+        if (on && !fast) v = sgs_divide(sum, D);
+        if (REV) v = in + v;
+        mine[(s & 1) * SGS_VALS] = v;
+        *cell = v;
+        if (on) last = v;
+    };
+    __syncthreads();
+    for (int t0 = 0; t0 < steps; t0 += SGS_C) {
+        double* const cur = chunks + ((t0 / SGS_C) % 3) * SGS_CHUNK + tid * SGS_P;
+        const int se = min(SGS_C, steps - t0);
+        for (int s0 = 0; s0 < se; s0 += 4) {
+            if (unsigned(t0 + s0 - high - 1) < unsigned(inside)) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    step(e, 0, cur + s0 + e, false);
+                    if (e < 3) sgs_step_barrier();
+                }
+            } else {
+                for (int s = s0; s < s0 + 4 && s < se; ++s) {
+                    if (unsigned(t0 + s - low) < unsigned(active)) step(s, t0 + s, cur + s, true);
+                    if (s < s0 + 3 && s + 1 < se) sgs_step_barrier();
+                }
+            }
+            if (s0 + 4 < se) sgs_step_barrier();
+        }
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(SGS_THREADS, 2) k_sgs_flow(const __grid_constant__ GridDev g, SolveState* st,
+                                                             const double* __restrict__ r, double* z, double* d0,
+                                                             double* d1, SgsFlow f, int mode) {
+    extern __shared__ __align__(16) double sgs_smem[];
+    double* const chunks = sgs_smem;
+    double* const vals = sgs_smem + 3 * SGS_CHUNK;
+    unsigned long long* const ring =
+        reinterpret_cast<unsigned long long*>(vals + 2 * SGS_VALS);  // on a 16-byte boundary
+    __shared__ int s_slot, s_fail;
     if (!gate(st->flags, mode)) return;
-    const int nt0 = (g.n[0] + SGS_T - 1) / SGS_T, nt1 = (g.n[1] + SGS_T - 1) / SGS_T,
-              nt2 = (g.n[2] + SGS_T - 1) / SGS_T;
-    const int lx = threadIdx.x % SGS_T, ly = (threadIdx.x / SGS_T) % SGS_T, lz = threadIdx.x / (SGS_T * SGS_T);
-    const int mine = lx + ly + lz;
-    const int sy = g.n[0], sz = g.n[0] * g.n[1];
-    const int slots = 2 * f.ntiles;
-    if (threadIdx.x == 0) s_slot = int(atomicAdd(f.ctl, 1u));
+    unsigned long long* const words = reinterpret_cast<unsigned long long*>(st->dsel ? d0 : d1);
+    const int units = f.nj * f.nk, slots = 2 * units;
+    const unsigned number = f.ctl[2 + units];
+    const int role = threadIdx.x < SGS_LINES ? 0 : (threadIdx.x < SGS_STEPPERS - 32 ? 1 : (threadIdx.x < SGS_STEPPERS ? 2 : 3));
+    if (threadIdx.x == 0) {
+        s_slot = int(atomicAdd(f.ctl, 1u));
+        s_fail = 0;
+    }
     __syncthreads();
     int slot = s_slot;
     while (slot < slots) {
-        // the next slot is taken now, its atomic overlapping this tile
+        // the next slot is taken now, its atomic overlapping this unit
         unsigned next_slot = 0;
         if (threadIdx.x == 0) next_slot = atomicAdd(f.ctl, 1u);
-        const bool reverse = slot >= f.ntiles;
-        const int tile = f.order[reverse ? slots - 1 - slot : slot];
-        const int tx = tile % nt0, ty = (tile / nt0) % nt1, tz = tile / (nt0 * nt1);
-        const int i = tx * SGS_T + lx, j = ty * SGS_T + ly, k = tz * SGS_T + lz;
-        const bool in = i < g.n[0] && j < g.n[1] && k < g.n[2];
-        const int c = in ? cell_idx(g, i, j, k) : 0;
-        double rv = 0.0, D = 1.0, y = 0.0;
-        if (in) {
-            const int m = diag_mask(g, i, j, k);
-            D = g.diag[m];
-            y = g.rdiag[m];
-            if (!reverse) rv = r[c];
-        }
-        if (threadIdx.x < 32) {
-            // lanes 0, 1, 2 wait on the x, y, z neighbour tile at once
-            const int lane = threadIdx.x;
-            int dep = -1;
-            unsigned need = 1u;
-            if (lane < 3) {
-                const int t = lane == 0 ? tx : (lane == 1 ? ty : tz);
-                const int n = lane == 0 ? nt0 : (lane == 1 ? nt1 : nt2);
-                const int stride = lane == 0 ? 1 : (lane == 1 ? nt0 : nt0 * nt1);
-                if (!reverse) {
-                    if (t > 0) dep = tile - stride;
-                } else if (tx + 1 == nt0 && ty + 1 == nt1 && tz + 1 == nt2) {
-                    if (lane == 0) dep = tile;  // the last tile of the forward order: its own forward sweep
-                } else if (t + 1 < n) {
-                    dep = tile + stride;
-                    need = 2u;
+        const bool reverse = slot >= units;
+        const int unit = f.order[reverse ? slots - 1 - slot : slot];
+        SgsUnit U;
+        U.jb = unit % f.nj;
+        U.kb = unit / f.nj;
+        U.j0 = U.jb * SGS_UJ;
+        U.k0 = U.kb * SGS_UK;
+        U.nj = min(SGS_UJ, g.n[1] - U.j0);
+        U.nk = min(SGS_UK, g.n[2] - U.k0);
+        const int steps = g.n[0] + U.nj + U.nk - 2;
+        const unsigned tag = kSgsTag | ((2u * number + (reverse ? 1u : 0u)) & 0x3ffffu);
+        if (reverse) {
+            if (threadIdx.x == 0) {
+                unsigned n = 0;
+                while (ld_acquire_u32(f.ctl + 2 + unit) == 0u) {
+                    ++n;
+                    const bool over = n > kSgsSpins;
+                    if (over) atomicExch(f.ctl + 1, 1u);
+                    if (over || ((n & 7u) == 0u && *(volatile const unsigned*)(f.ctl + 1) != 0u)) {
+                        s_fail = 1;
+                        break;
+                    }
+                    if (n > 256u) __nanosleep(64);
                 }
             }
-            const bool ok = __all_sync(0xffffffffu, dep < 0 || sgs_wait(f.ctl, dep, need));
-            if (lane == 0) s_ok = ok;
+            __syncthreads();
+            if (!s_fail) {
+                if (role == 0) sgs_lines<true>(g, U, steps, chunks, vals);
+                else if (role == 1) sgs_faces<true>(g, f, U, steps, words, tag, vals, ring, &s_fail);
+                else if (role == 2) sgs_send<true>(g, f, U, steps, words, tag, vals);
+                else sgs_move<true>(g, U, steps, r, z, chunks);
+            }
+        } else {
+            if (role == 0) sgs_lines<false>(g, U, steps, chunks, vals);
+            else if (role == 1) sgs_faces<false>(g, f, U, steps, words, tag, vals, ring, &s_fail);
+            else if (role == 2) sgs_send<false>(g, f, U, steps, words, tag, vals);
+            else sgs_move<false>(g, U, steps, r, z, chunks);
         }
         __syncthreads();
-        if (!s_ok) {
+        if (s_fail) {
             if (threadIdx.x == 0) {
                 atomicExch(f.ctl + 1, 1u);
                 st->status = RB200_EXECUTION;
@@ -460,49 +769,11 @@ __global__ void __launch_bounds__(SGS_THREADS) k_sgs_flow(GridDev g, SolveState*
             }
             return;
         }
-        double* const me = &zs[lz + 1][ly + 1][lx + 1];
-        if (!reverse) {
-            if (in) {
-                if (c == 0) *me = __ldcg(z);  // the gauge row keeps its value
-                if (lx == 0 && i > 0) zs[lz + 1][ly + 1][0] = __ldcg(z + c - 1);
-                if (ly == 0 && j > 0) zs[lz + 1][0][lx + 1] = __ldcg(z + c - sy);
-                if (lz == 0 && k > 0) zs[0][ly + 1][lx + 1] = __ldcg(z + c - sz);
-            }
-            __syncthreads();
-            for (int l = 0; l < 3 * SGS_T - 2; ++l) {
-                if (in && mine == l && c != 0) {
-                    double value = rv;
-                    if (i > 0) value += g.weight[0] * zs[lz + 1][ly + 1][lx];
-                    if (j > 0) value += g.weight[1] * zs[lz + 1][ly][lx + 1];
-                    if (k > 0) value += g.weight[2] * zs[lz][ly + 1][lx + 1];
-                    *me = div_diag(value, D, y);
-                }
-                __syncthreads();
-            }
-        } else {
-            if (in) {
-                *me = __ldcg(z + c);
-                if (lx == SGS_T - 1 && i + 1 < g.n[0]) zs[lz + 1][ly + 1][SGS_T + 1] = __ldcg(z + c + 1);
-                if (ly == SGS_T - 1 && j + 1 < g.n[1]) zs[lz + 1][SGS_T + 1][lx + 1] = __ldcg(z + c + sy);
-                if (lz == SGS_T - 1 && k + 1 < g.n[2]) zs[SGS_T + 1][ly + 1][lx + 1] = __ldcg(z + c + sz);
-            }
-            __syncthreads();
-            for (int l = 3 * SGS_T - 3; l >= 0; --l) {
-                if (in && mine == l && c != 0) {
-                    double correction = 0.0;
-                    if (i + 1 < g.n[0]) correction += g.weight[0] * zs[lz + 1][ly + 1][lx + 2];
-                    if (j + 1 < g.n[1]) correction += g.weight[1] * zs[lz + 1][ly + 2][lx + 1];
-                    if (k + 1 < g.n[2]) correction += g.weight[2] * zs[lz + 2][ly + 1][lx + 1];
-                    *me = *me + div_diag(correction, D, y);
-                }
-                __syncthreads();
-            }
-        }
-        if (in && c != 0) __stcg(z + c, *me);
-        __syncthreads();
         if (threadIdx.x == 0) {
-            __threadfence();
-            st_release_u32(f.ctl + 2 + tile, reverse ? 2u : 1u);
+            if (!reverse) {
+                __threadfence();
+                st_release_u32(f.ctl + 2 + unit, 1u);
+            }
             s_slot = int(next_slot);
         }
         __syncthreads();
@@ -510,13 +781,14 @@ __global__ void __launch_bounds__(SGS_THREADS) k_sgs_flow(GridDev g, SolveState*
     }
 }
 
-// r.z after a lexicographic SGS application, then the preconditioner decision.
 __global__ void __launch_bounds__(EW) k_sgs_dot(GridDev g, SolveState* st, const double* __restrict__ r,
                                                 const double* __restrict__ z, int mode, Partials part,
                                                 rb200_trace* trace, unsigned* sgs_ctl, int sgs_words) {
     __shared__ BlockReduce<1, 0> sm;
     // the sweep kernel before this one has ended: its queue starts over
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < sgs_words; t += gridDim.x * blockDim.x) sgs_ctl[t] = 0u;
+    // and its number moves on (the word after the states)
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t <= sgs_words; t += gridDim.x * blockDim.x)
+        sgs_ctl[t] = t < sgs_words ? 0u : sgs_ctl[t] + 1u;
     if (!gate(st->flags, mode)) return;
     Neu acc;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < g.cells; c += gridDim.x * blockDim.x)
@@ -763,9 +1035,9 @@ static TmaMaps make_maps(const GridDev& g, const double* z, const double* d0, co
 
 // One lexicographic SGS application: both sweeps in one launch, then r.z.
 static int launch_sgs(const GridDev& g, const Bufs& B, int mode, cudaStream_t s) {
-    k_sgs_flow<<<B.sgs.blocks, SGS_THREADS, 0, s>>>(g, B.st, B.r, B.z, B.sgs, mode);
+    k_sgs_flow<<<B.sgs.blocks, SGS_THREADS, kSmemSgs, s>>>(g, B.st, B.r, B.z, B.d0, B.d1, B.sgs, mode);
     k_sgs_dot<<<ew_blocks(g.cells), EW, 0, s>>>(g, B.st, B.r, B.z, mode, B.part, B.trace, B.sgs.ctl,
-                                                B.sgs.ntiles + 2);
+                                                B.sgs.nj * B.sgs.nk + 2);
     return 2;
 }
 
@@ -970,33 +1242,32 @@ static bool persistent_graphs_supported(PcgSolver& solver) {
     return supported;
 }
 
-// The lexicographic SGS queue: tile ids in wave order, the zeroed state
+// The lexicographic SGS queue: unit ids in wave order, the zeroed state
 // words, and the sweep kernel's resident block count.
 int PcgSolver::sgs_setup() {
-    const int nt0 = (g_.n[0] + SGS_T - 1) / SGS_T, nt1 = (g_.n[1] + SGS_T - 1) / SGS_T,
-              nt2 = (g_.n[2] + SGS_T - 1) / SGS_T;
+    sgs_.nj = (g_.n[1] + SGS_UJ - 1) / SGS_UJ;
+    sgs_.nk = (g_.n[2] + SGS_UK - 1) / SGS_UK;
     std::vector<int> order;
-    order.reserve(size_t(nt0) * nt1 * nt2);
-    for (int w = 0; w <= nt0 + nt1 + nt2 - 3; ++w)
-        for (int tz = 0; tz < nt2; ++tz)
-            for (int ty = 0; ty < nt1; ++ty) {
-                const int tx = w - ty - tz;
-                if (tx >= 0 && tx < nt0) order.push_back(tx + nt0 * (ty + nt1 * tz));
-            }
-    sgs_.ntiles = int(order.size());
+    order.reserve(size_t(sgs_.nj) * sgs_.nk);
+    for (int w = 0; w <= sgs_.nj + sgs_.nk - 2; ++w)
+        for (int kb = std::max(0, w - sgs_.nj + 1); kb <= std::min(w, sgs_.nk - 1); ++kb)
+            order.push_back(w - kb + sgs_.nj * kb);
+    const size_t units = order.size(), words = units + 3;
     int* d_order = nullptr;
-    RB200_CUDA(cudaMalloc(&d_order, order.size() * sizeof(int)));
+    RB200_CUDA(cudaMalloc(&d_order, units * sizeof(int)));
     sgs_.order = d_order;
-    RB200_CUDA(cudaMalloc(&sgs_.ctl, (order.size() + 2) * sizeof(unsigned)));
-    bytes_ += order.size() * sizeof(int) + (order.size() + 2) * sizeof(unsigned);
-    RB200_CUDA(cudaMemcpyAsync(d_order, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice, stream_));
-    RB200_CUDA(cudaMemsetAsync(sgs_.ctl, 0, (order.size() + 2) * sizeof(unsigned), stream_));
+    RB200_CUDA(cudaMalloc(&sgs_.ctl, words * sizeof(unsigned)));
+    bytes_ += units * sizeof(int) + words * sizeof(unsigned);
+    RB200_CUDA(cudaMemcpyAsync(d_order, order.data(), units * sizeof(int), cudaMemcpyHostToDevice, stream_));
+    RB200_CUDA(cudaMemsetAsync(sgs_.ctl, 0, words * sizeof(unsigned), stream_));
+    for (double* d : d_) RB200_CUDA(cudaMemsetAsync(d, 0, size_t(g_.cells) * sizeof(double), stream_));
     RB200_CUDA(cudaStreamSynchronize(stream_));
     int dev = 0, sms = 0, per_sm = 0;
     RB200_CUDA(cudaGetDevice(&dev));
     RB200_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    RB200_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sgs_flow, SGS_THREADS, 0));
-    sgs_.blocks = int(std::min<long long>(2ll * sgs_.ntiles, std::max(1ll, (long long)sms * per_sm)));
+    RB200_CUDA(cudaFuncSetAttribute(k_sgs_flow, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemSgs)));
+    RB200_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sgs_flow, SGS_THREADS, kSmemSgs));
+    sgs_.blocks = int(std::min<long long>(2ll * (long long)units, std::max(1ll, (long long)sms * per_sm)));
     return RB200_OK;
 }
 

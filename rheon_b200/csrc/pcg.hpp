@@ -64,13 +64,14 @@ struct GridBarrier {
 };
 
 // Work queue of the lexicographic SGS preconditioner (one launch per
-// application, forward and reverse sweep): the 8^3 tiles in wave order and
-// one state word per tile. The word block is zeroed by the r.z kernel that
-// follows every application.
+// application, forward and reverse sweep): the units of 16 x 16 lines along x
+// in wave order and one state word per unit. The queue and the states are
+// zeroed by the r.z kernel that follows every application, which also counts
+// the applications.
 struct SgsFlow {
-    const int* order = nullptr;  // tile ids (tx + ntx (ty + nty tz)), waves tx + ty + tz ascending
-    unsigned* ctl = nullptr;     // [0] next queue slot, [1] abort, [2 + tile] 1 forward done, 2 reverse done
-    int ntiles = 0;
+    const int* order = nullptr;  // unit ids (jb + nj kb), waves jb + kb ascending
+    unsigned* ctl = nullptr;     // [0] next queue slot, [1] abort, [2 + unit] forward done, then the application's number
+    int nj = 0, nk = 0;          // units along y and z
     int blocks = 0;              // resident blocks of the sweep kernel
 };
 
