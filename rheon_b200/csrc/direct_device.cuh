@@ -17,6 +17,20 @@ __host__ __device__ __forceinline__ int dct_row_pitch(int neP, int noP) { return
 
 enum DctOp : int { DCT_FORWARD = 0, DCT_INVERSE = 1, DCT_SOLVE = 2 };
 
+// Two floats as one register pair, and the pair's multiply-add (each rounded as
+// fmaf rounds it).
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
 // The register block's inner product over one staged table chunk: RM outputs x
 // 4 lines per thread. Lines along x (ROW) keep their elements contiguous in
 // shared memory and are read four contraction steps at a time; other lines are
@@ -24,6 +38,11 @@ enum DctOp : int { DCT_FORWARD = 0, DCT_INVERSE = 1, DCT_SOLVE = 2 };
 template <int RM, bool ROW>
 __device__ __forceinline__ void dct_chunk(float (&acc)[RM][4], const float* __restrict__ sT, int mP,
                                           const float* __restrict__ sX, int pitch, int lstep, int rows) {
+    unsigned long long p[RM / 2][4];
+#pragma unroll
+    for (int r = 0; r < RM / 2; ++r)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) p[r][j] = pack2(acc[2 * r][j], acc[2 * r + 1][j]);
 #pragma unroll 1
     for (int k = 0; k < rows; k += 4) {
         float b[4][4];  // [step][line]
@@ -48,31 +67,31 @@ __device__ __forceinline__ void dct_chunk(float (&acc)[RM][4], const float* __re
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            float a[RM];
+            unsigned long long a[RM / 2], w[4];
             const float* t = sT + (k + u) * mP;
             if (RM % 4 == 0) {
 #pragma unroll
                 for (int r = 0; r < RM / 4; ++r) {
-                    const float4 v = *reinterpret_cast<const float4*>(t + 4 * r);
-                    a[4 * r] = v.x;
-                    a[4 * r + 1] = v.y;
-                    a[4 * r + 2] = v.z;
-                    a[4 * r + 3] = v.w;
-                }
-            } else {
-#pragma unroll
-                for (int r = 0; r < RM / 2; ++r) {
-                    const float2 v = *reinterpret_cast<const float2*>(t + 2 * r);
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(t + 4 * r);
                     a[2 * r] = v.x;
                     a[2 * r + 1] = v.y;
                 }
+            } else {
+#pragma unroll
+                for (int r = 0; r < RM / 2; ++r) a[r] = *reinterpret_cast<const unsigned long long*>(t + 2 * r);
             }
 #pragma unroll
-            for (int r = 0; r < RM; ++r)
+            for (int j = 0; j < 4; ++j) w[j] = pack2(b[u][j], b[u][j]);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[r][j] = fmaf(a[r], b[u][j], acc[r][j]);
+            for (int r = 0; r < RM / 2; ++r)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) fma2(p[r][j], a[r], w[j]);
         }
     }
+#pragma unroll
+    for (int r = 0; r < RM / 2; ++r)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) unpack2(p[r][j], acc[2 * r][j], acc[2 * r + 1][j]);
 }
 
 // Both halves of a transform from the staged tile (even part in the first neP
@@ -117,11 +136,14 @@ __device__ __forceinline__ void dct_product(float (&ae)[RM][4], float (&ao)[RM][
     }
 }
 
-// One tile of 32 nb lines (k_dct, k_b_dct). Bound by the FP32 pipes: n / 2
-// multiply-adds per element and transform against 8 bytes moved, and the tables
-// come from L2. A whole line set per block (a 64 KB tile at n = 256) keeps the
-// element traffic at one read and one write a pass; 8 x 4 outputs a thread
-// leave 3 shared-memory wavefronts for 32 multiply-adds a warp.
+// One tile of 32 nb lines (k_dct, k_b_dct). Bound by shared-memory reads and the
+// FP32 pipes: n / 2 multiply-adds per element and transform against 8 bytes
+// moved, and the tables come from L2. A whole line set per block (a 64 KB tile
+// at n = 256) keeps the element traffic at one read and one write a pass; 8 x 4
+// outputs a thread take three 16-byte reads for 32 multiply-adds, issued two at
+// a time (paired: the six transforms of 256^3 920 us against 990 one at a time,
+// in a step 3436 against 3610). 8 x 8 outputs, three quarters of the reads but
+// half the warps, took 5% longer on a step of 256^3 and 7% on one of 128^3.
 // The whole lines of the tile are staged in shared
 // memory before anything is written, so src and dst may be the same array.
 // `cold`: read src64 instead of src.
