@@ -383,11 +383,10 @@ __global__ void __launch_bounds__(EW) k_mg_update(GridDev g, SolveState* st, dou
 // which comes after every other forward sweep.
 //
 // us per iteration of a solve, tiles of 8^3 cells with a block barrier for each
-// of their 22 hyperplanes / this: 32^3 138 / 83, 63x48x37 226 / 108, 96^3
-// 453 / 207, 256x20x20 417 / 124. Units of 16 x 16 lines took 113, 222 and 148
-// for the last three (two line warps to a scheduler), fetching the faces 7
-// steps ahead 120, 238 and 130 (a unit that catches up with its neighbour polls
-// for every word in flight).
+// of their 22 hyperplanes / this: 32^3 138 / 83, 63x48x37 226 / 102, 96^3
+// 453 / 208, 256x20x20 417 / 124. Units of 16 x 16 lines took 113, 222 and 148
+// for the last three (two line warps to a scheduler); with face words in flight
+// left as they were after a wait, each to be waited for in turn, 108, 207 and 124.
 //
 // Every wait is bounded: a wait that runs out raises the abort word, which
 // ends every other wait, and marks the solve as failed (execution error).
@@ -398,7 +397,7 @@ constexpr int SGS_LINES = SGS_UJ * SGS_UK;
 constexpr int SGS_MOVERS = 64;                 // threads that move the chunks
 constexpr int SGS_STEPPERS = SGS_LINES + 64;   // the lines and the faces' two warps: they share the step barrier
 constexpr int SGS_THREADS = SGS_STEPPERS + SGS_MOVERS;
-constexpr int SGS_AHEAD = 5;                   // steps between a face word's load and its use
+constexpr int SGS_AHEAD = 6;                   // steps between a face word's load and its use
 constexpr int SGS_VP = SGS_UJ + 2;             // pitch of the step values
 constexpr int SGS_VALS = (SGS_UK + 1) * SGS_VP;
 constexpr int SGS_CHUNK = SGS_LINES * SGS_P;
@@ -480,7 +479,8 @@ __device__ __noinline__ bool sgs_poll(const unsigned long long* p, unsigned tag,
 // The incoming faces' warp of a unit: lane q fetches line q of the y face, lane
 // 16 + q of the z face, one step of the unit at a time. The words come through
 // asynchronous copies, since a load into registers would be waited for at the
-// next branch; a word that came too early is polled for.
+// next branch; a copy that came before its word is polled for, and those behind
+// it are made again.
 template <bool REV>
 __device__ __forceinline__ void sgs_faces(const GridDev& g, const SgsFlow& f, const SgsUnit& U, int steps,
                                           const unsigned long long* words, unsigned tag, double* vals,
@@ -514,11 +514,15 @@ __device__ __forceinline__ void sgs_faces(const GridDev& g, const SgsFlow& f, co
     auto deliver = [&](int t) {
         const bool want = wanted(t);
         const bool ok = !want || (unsigned(lo >> 32) == tag && unsigned(hi >> 32) == tag);
-        if (!__all_sync(0xffffffffu, ok) && !dead && !sgs_poll(want ? word(t) : words, tag, want, f.ctl, &lo, &hi)) {
-            dead = true;
-            if (lane == 0) {
-                atomicExch(f.ctl + 1, 1u);
-                *s_fail = 1;
+        if (!__all_sync(0xffffffffu, ok) && !dead) {
+            if (sgs_poll(want ? word(t) : words, tag, want, f.ctl, &lo, &hi)) {
+                for (int e = 1; e < SGS_AHEAD - 1; ++e) fetch(t + e);  // those in flight came too early as well
+            } else {
+                dead = true;
+                if (lane == 0) {
+                    atomicExch(f.ctl + 1, 1u);
+                    *s_fail = 1;
+                }
             }
         }
         if (want) to[((t + 1) & 1) * SGS_VALS] = __hiloint2double(int(unsigned(hi)), int(unsigned(lo)));
