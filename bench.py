@@ -41,6 +41,9 @@ WORKLOAD = ("fixed-box carrier step: {n}^3 cells, {storage} faces, random-Fourie
             "{method} to rel residual 1e-8")
 METRIC = "cell-steps/s at rel. residual 1e-8 (plain f64 GPU path)"
 UNIT = "cell-steps/s"
+# algorithmic bytes a cell of a mixed outer iteration: five FP32 transform
+# passes (44) and the FP64 refinement (24)
+MIXED_BYTES = 68
 MAXF = 1.7976931348623157e308
 
 
@@ -252,9 +255,9 @@ def run_batched(args, local, flush):
         launches += out[0][1].kernel_launches
         solve_ms += out[0][1].pressure_ms
         # the algorithmic byte model of a mixed step, summed over instances:
-        # 130N per outer iteration (FP32 V(2,2), levels summed, + FP64 defect
-        # and accumulation) and 5 F s + 16N for advection, RHS and correction
-        model_bytes += sum(it * 130 * c + 5 * f * 4 + 16 * c for it, c, f in zip(its, cells, faces_total))
+        # MIXED_BYTES N per outer iteration and 5 F s + 16N for advection, RHS
+        # and correction
+        model_bytes += sum(it * MIXED_BYTES * c + 5 * f * 4 + 16 * c for it, c, f in zip(its, cells, faces_total))
     hbm, hbm_kind = peaks()
     achieved = model_bytes / (total_ms / 1e3) / 1e9
     ms_step = total_ms / args.batched_steps
@@ -271,10 +274,10 @@ def run_batched(args, local, flush):
         "iterations_max": max(iters),
         "graph_launches_per_batched_step": 1,
         "kernels_per_batched_step": launches / args.batched_steps,
-        "dtype": "mixed (f32 faces and V-cycles, f64 residual/accumulation/coarse solve)",
+        "dtype": "mixed (f32 faces and preconditioner, f64 residual and accumulation)",
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "peak_kind": hbm_kind, "unit": "GB/s",
                      "frac": achieved / hbm, "bytes_per_batched_step": model_bytes / args.batched_steps,
-                     "model": "sum over instances of 130N per outer iteration + 5Fs + 16N per step"},
+                     "model": f"sum over instances of {MIXED_BYTES}N per outer iteration + 5Fs + 16N per step"},
     }
     batch.close()
     # the same boxes as separate resident carriers launched together
@@ -387,8 +390,8 @@ def run_batch_profile(args, local):
 def run_mixed_large(args, local, flush, n):
     """The mixed-precision carrier at n^3 (random-Fourier state generated on the
     device, CFL 0.5, rel. residual 1e-8): device-timed steps and the step's
-    roofline under the algorithmic byte model (130N per outer iteration,
-    5 F s + 16N per step, s = 4)."""
+    roofline under the algorithmic byte model (MIXED_BYTES N per outer
+    iteration, 5 F s + 16N per step, s = 4)."""
     import torch
 
     import rheon_b200 as R
@@ -418,7 +421,7 @@ def run_mixed_large(args, local, flush, n):
     sim.close()
     cells = n ** 3
     faces = 3 * n * n * (n + 1)
-    step_bytes = statistics.mean(its) * 130 * cells + 5 * faces * 4 + 16 * cells
+    step_bytes = statistics.mean(its) * MIXED_BYTES * cells + 5 * faces * 4 + 16 * cells
     hbm, hbm_kind = peaks()
     ach = step_bytes / (ms / steps / 1e3) / 1e9
     return {"workload": f"mixed carrier step at {n}^3, random-Fourier init, CFL 0.5, rel 1e-8",
@@ -426,7 +429,7 @@ def run_mixed_large(args, local, flush, n):
             "pressure_ms_per_step": solve / steps, "iterations_per_step": statistics.mean(its),
             "roofline": {"bound": "hbm", "achieved": ach, "peak": hbm, "peak_kind": hbm_kind, "unit": "GB/s",
                          "frac": ach / hbm, "bytes_per_step": step_bytes,
-                         "model": "130N per outer iteration + 5Fs + 16N per step"}}
+                         "model": f"{MIXED_BYTES}N per outer iteration + 5Fs + 16N per step"}}
 
 
 def run_serving(args, local):
@@ -523,8 +526,8 @@ def run_solve_only(args, local):
 
 def run_buoyant_blob(args, local):
     """Mixed precision on a buoyant Gaussian blob: the mixed carrier (FP32
-    faces and advection, FP32 multigrid V(2,2) inside FP64 flexible CG, FP64
-    residual, accumulation and coarsest solve) to relative residual 1e-10,
+    faces and advection, the FP32 direct preconditioner inside FP64 iterative
+    refinement) to relative residual 1e-10,
     stepped in lockstep with the f64 carrier (f64 faces and advection,
     Jacobi-PCG to 1e-10: the path that tracks the oracle per iteration). Both
     advect a passive density blob (sigma 20 cells, peak 1, centred at
@@ -820,7 +823,7 @@ def run_box_flux(args, local, with_cpu):
     """Box-flux projection (src/box_flux.rs:213-397) at n^3 on the unit cube: a
     seeded random-Fourier provisional field with a 0.5 m/s through-flow along
     x imposed on the sides, projected with the reference's default pressure
-    method (Jacobi-PCG) and with the mixed-precision multigrid. Device time of
+    method (Jacobi-PCG) and with the mixed-precision method. Device time of
     a whole projection (CUDA events on the workspace's stream, host polls of
     the solve included), the fused passes' own times inside it, the same call
     on pinned host arrays, and the oracle's projection on one host core."""
@@ -925,7 +928,7 @@ def run_box_flux_step(args, local, with_cpu):
     """Simulation::step_with_box_flux (src/simulation.rs:551-579) on the resident
     carrier at n^3 on the unit cube: the random-Fourier state, a smoke source in
     the box's centre, a uniform body force and a 0.5 m/s x through-flow, on the
-    mixed carrier (FP32 multigrid) and the f32 Jacobi-PCG carrier (rel 1e-8).
+    mixed carrier and the f32 Jacobi-PCG carrier (rel 1e-8).
     Wall time per step (the step is host-driven and synchronous), and the
     oracle's step on one host core."""
     import torch
@@ -1069,6 +1072,10 @@ def run_ours(args, world, rank, local):
         # reads z, d_old and writes d_new, phase 2 reads d, p, r and writes
         # p, r, z)
         roof_kernel, roof_bytes, roof_ms = "k_jacobi_persistent (one PCG iteration)", 88 * cells, iter_ms
+        if method == R.PressureImplementation.JACOBI_PCG_V1 and ((args.n + 31) // 32) ** 2 * ((args.n + 15) // 16) <= 148:
+            # boxes of at most 148 bricks of 32 x 16 x 32 cells keep the
+            # direction and the residual on the chip: only p crosses (16N)
+            roof_kernel, roof_bytes = "k_jacobi_resident (one PCG iteration)", 16 * cells
         other_ms = sim.profile(1, launches_prof) if method != R.PressureImplementation.MG_MIXED else 0.0
     except R.SimulationError:
         pass
@@ -1129,16 +1136,14 @@ def run_ours(args, world, rank, local):
                               "vs_plain_f64": vvalue / value}
             if vcfg.implementation == R.PressureImplementation.MG_MIXED:
                 # whole-step roofline under the algorithmic byte model of a
-                # mixed outer cycle: an FP32 V(2,2) with levels summed (about
-                # 82N) plus the FP64 defect and accumulation (48N) = 130N per
-                # outer iteration, and the step's non-iterative traffic
+                # mixed outer iteration and the step's non-iterative traffic
                 # (advection, RHS, correction: 5 F s + 16N with s = 4 bytes)
                 faces_total = sum(g.face_len(d) for d in range(3))
-                step_bytes = statistics.mean(vit) * 130 * cells + 5 * faces_total * 4 + 16 * cells
+                step_bytes = statistics.mean(vit) * MIXED_BYTES * cells + 5 * faces_total * 4 + 16 * cells
                 ach = step_bytes / (vms / args.steps / 1e3) / 1e9
                 variants[name]["roofline"] = {"bound": "hbm", "achieved": ach, "peak": hbm, "unit": "GB/s",
                                               "frac": ach / hbm, "bytes_per_step": step_bytes,
-                                              "model": "130N per outer iteration + 5Fs + 16N per step"}
+                                              "model": f"{MIXED_BYTES}N per outer iteration + 5Fs + 16N per step"}
             vs.close()
 
     mixed256 = None
@@ -1167,7 +1172,7 @@ def run_ours(args, world, rank, local):
         "config": {
             "workload": WORKLOAD.format(n=args.n, storage=args.storage,
                                         method={"jacobi": "Jacobi-PCG", "rbsgs": "RB-SGS-PCG", "sgs": "SGS-PCG (v1)",
-                                                "mixed": "FP32-multigrid FCG"}[args.method]),
+                                                "mixed": "FP32-direct refinement"}[args.method]),
             "cells": cells,
             "parallelism": f"replicas x{world} (independent boxes, no collective)",
             "l2": "256 MB buffer written between timed steps; per-step working set > 126 MB L2",

@@ -72,9 +72,10 @@ typedef enum rb200_status {
 /* Pressure methods. JACOBI_PCG_V1 reproduces "jacobi-pcg-v1"
  * (src/pressure.rs:7-29). SGS_PCG_V1 reproduces the exact lexicographic
  * "sgs-pcg-v1" sweep order. RBSGS_PCG is the device-native red-black symmetric
- * Gauss-Seidel preconditioner (new). MG_MIXED is flexible CG with an FP32
- * geometric multigrid V(2,2) preconditioner, FP64 residual/accumulation and an
- * FP64 coarse solve (new). */
+ * Gauss-Seidel preconditioner (new). MG_MIXED is FP64 iterative refinement with
+ * an FP32 direct preconditioner (fast diagonalisation); grids with an axis
+ * beyond 512 cells, all axes of at most 8 or a condition beyond 1e9 take FP64
+ * flexible CG with an FP32 geometric multigrid V(2,2) preconditioner (new). */
 typedef enum rb200_method {
     RB200_JACOBI_PCG_V1 = 0,
     RB200_SGS_PCG_V1 = 1,
@@ -417,8 +418,8 @@ RB200_API int rb200_carriers_step(rb200_carrier* const* carriers, size_t count, 
                                   rb200_step_report* reports, int* statuses);
 /* ------------------------------------------------- packed batch of carriers
  * Many independent fixed boxes of uneven sizes stepped together with the
- * mixed-precision pressure method (f32 faces, FP32 multigrid V(2,2) inside
- * FP64 flexible CG). No counterpart in the reference, which steps one box at a
+ * mixed-precision pressure method (f32 faces, an FP32 preconditioner inside an
+ * FP64 iteration). No counterpart in the reference, which steps one box at a
  * time (src/simulation.rs:812-1403); every instance follows that step owner's
  * order, gates and transactional commit. All instances live in one device
  * arena, every stage of the step is one launch over all of them, and a step of

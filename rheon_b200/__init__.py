@@ -548,8 +548,9 @@ class CarrierConfig:
     @staticmethod
     def mixed(**kw) -> "CarrierConfig":
         """The mixed-precision carrier: FP32 faces and FP32 advection
-        arithmetic, FP32 multigrid V(2,2) smoothing inside FP64 flexible CG
-        (FP64 residual, pressure accumulation and coarsest solve)."""
+        arithmetic, an FP32 direct preconditioner (multigrid on the grids
+        it does not cover) inside an FP64 iteration (FP64 residual and
+        pressure accumulation)."""
         kw.setdefault("storage", "f32")
         kw.setdefault("implementation", PressureImplementation.MG_MIXED)
         kw.setdefault("fp32_advection", True)
@@ -755,9 +756,9 @@ def step_all(sims: Sequence["CarrierSimulation"], params: Sequence[StepParams]):
 class BatchedCarriers:
     """Many independent fixed boxes of uneven sizes stepped together: every
     stage of the step is one launch over all instances and one step of the
-    batch is one CUDA graph (mixed precision: f32 faces, FP32 multigrid inside
-    FP64 flexible CG). Each instance's results are the same bits as in a batch
-    of its own."""
+    batch is one CUDA graph (mixed precision: f32 faces, an FP32
+    preconditioner inside an FP64 iteration). Each instance's results are the
+    same bits as in a batch of its own."""
 
     def __init__(self, grids: Sequence[GridGeometry], config: Optional[CarrierConfig] = None):
         config = config or CarrierConfig.mixed()

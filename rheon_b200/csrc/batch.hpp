@@ -2,8 +2,8 @@
 // mixed-precision pressure method (new; the reference steps one box at a time,
 // src/simulation.rs:812-1403).
 //
-// Every instance keeps its own accepted state, solver vectors and multigrid
-// hierarchy in one device arena; a device table describes them. Each kernel of
+// Every instance keeps its own accepted state, solver vectors and preconditioner
+// in one device arena; a device table describes them. Each kernel of
 // the step is ONE launch over all instances: a launch gives every instance a
 // contiguous range of blocks (its span), found by a binary search over the
 // ranges passed in the kernel's parameters, and every body works on its

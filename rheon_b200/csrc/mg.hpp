@@ -1,5 +1,6 @@
 // Mixed-precision geometric multigrid preconditioner for the sealed-box
-// pressure system (new; the reference has no multigrid).
+// pressure system (new; the reference has no multigrid), for the grids that the
+// direct preconditioner (direct.hpp) does not cover.
 //
 // One V(2,2) cycle in FP32 on a hierarchy of cell-centred grids: symmetric
 // red-black Gauss-Seidel smoothing (red then black before, black then red

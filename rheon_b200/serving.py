@@ -114,7 +114,7 @@ def merge_completions(per_rank: Sequence[Sequence[Completion]]) -> List[Completi
 
 def carrier_bytes_estimate(edge: int, config: CarrierConfig) -> int:
     """Device bytes of one carrier (three face buffers, solver vectors, the
-    FP32 multigrid hierarchy), before it is created."""
+    FP32 preconditioner's), before it is created."""
     n = edge ** 3
     faces = 3 * edge * edge * (edge + 1)
     elem = 4 if config.storage == "f32" else 8
