@@ -1337,7 +1337,7 @@ int rb200_batch_create(const rb200_grid* grids, size_t count, const rb200_batch_
             R.r32 = reinterpret_cast<float*>(take(size_t(g.cells) * 4));
             refs.push_back(R);
             DctJob J[5];
-            direct_jobs(*B->dct_tables[size_t(table_of[i])], g, I.b, R.r32, R.z, J);
+            direct_jobs(*B->dct_tables[size_t(table_of[i])], g, I.b, R.r32, R.z, false, J);
             for (int q = 0; q < 5; ++q) {
                 // an instance's tiles depend on its own grid only
                 J[q].nb = std::max(1, (DCT_THREADS / 32) / J[q].A.MB);

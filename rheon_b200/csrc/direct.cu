@@ -139,7 +139,8 @@ size_t direct_job_smem(const DctJob& J) {
     return (2 * size_t(DCT_KB) * J.A.mP + tc + tile) * sizeof(float);
 }
 
-void direct_jobs(const DctTables& T, const GridDev& g, const double* b, const float* r32, float* z, DctJob (&jobs)[5]) {
+void direct_jobs(const DctTables& T, const GridDev& g, const double* b, const float* r32, float* z, bool alone,
+                 DctJob (&jobs)[5]) {
     const int axis_of[5] = {0, 1, 2, 1, 0};
     for (int q = 0; q < 5; ++q) {
         DctJob& J = jobs[q];
@@ -156,6 +157,15 @@ void direct_jobs(const DctTables& T, const GridDev& g, const double* b, const fl
         J.lam1 = T.axis[1].lam;
         // Tiles as wide as eight warps allow while two blocks per SM all have
         // one; narrower ones on small grids.
+        // Few lines leave the SMs without warps to hide the shared reads: below
+        // six warps an SM a thread takes 4 outputs, and a transform up to twice
+        // the warps (us per solve of two iterations, 6 or 8 outputs / 4: 64^3
+        // 175 / 148, 90x75x63 279 / 227, 96^3 206 / 195, 112^3 266 / 247; at
+        // seven warps an SM 128^3 302 / 302, 512x64x64 414 / 448).
+        if (alone && J.A.RM > 4 && (J.lines + 31) / 32 * J.A.MB < 6 * 148 && J.A.mP % 16 == 0 && J.A.mP <= 128) {
+            J.A.RM = 4;
+            J.A.MB = J.A.mP / 16;
+        }
         J.nb = std::max(1, 8 / J.A.MB);
         while (J.nb > 1 && (J.lines + 32 * J.nb - 1) / (32 * J.nb) < 2 * 148) --J.nb;
         J.tiles = (J.lines + 32 * J.nb - 1) / (32 * J.nb);
@@ -213,7 +223,7 @@ int DirectSolver::enqueue_seed(const GridDev& g, SolveState* st, const double* b
 int DirectSolver::enqueue_iteration(const GridDev& g, SolveState* st, const double* b, double* p, double* p2,
                                     Partials part, rb200_trace* trace, cudaStream_t s) const {
     DctJob jobs[5];
-    direct_jobs(tables_, g, b, r32_, z_, jobs);
+    direct_jobs(tables_, g, b, r32_, z_, true, jobs);
     auto go = [&](void (*kernel)(const DctJob, const SolveState*), const DctJob& J) {
         pdl_launch(kernel, dim3(J.tiles), dim3(32 * J.A.MB * J.nb), direct_job_smem(J), s, J,
                    static_cast<const SolveState*>(st));

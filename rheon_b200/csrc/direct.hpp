@@ -80,8 +80,10 @@ bool direct_supported(const GridDev& g);
 
 // The passes of one application, in order: x, y forward, z forward, division
 // and inverse, y, x inverse. r32 -> z through `z` in place; b is read instead
-// of r32 by the first pass of a cold solve.
-void direct_jobs(const DctTables& T, const GridDev& g, const double* b, const float* r32, float* z, DctJob (&jobs)[5]);
+// of r32 by the first pass of a cold solve. `alone`: the grid has the chip to
+// itself (an instance of a batch does not).
+void direct_jobs(const DctTables& T, const GridDev& g, const double* b, const float* r32, float* z, bool alone,
+                 DctJob (&jobs)[5]);
 size_t direct_job_smem(const DctJob& J);
 
 class DirectSolver {

@@ -95,3 +95,10 @@ def test_seeded_direct_solve(n):
 def test_boxes_at_and_outside_the_direct_solves_limits_converge(n, h):
     # longer than 512 cells, no hierarchy, a condition of 2e7
     check(n, h, 1e-8, 7)
+
+
+@pytest.mark.parametrize("n", [(90, 130, 130), (128, 120, 128), (56, 170, 168)], ids=lambda n: "x".join(map(str, n)))
+def test_direct_solve_where_a_thread_takes_more_outputs(n):
+    # more than six warps an SM: 6 or 8 outputs a thread on the axes of 90, 128
+    # and 56 cells, 4 outputs on boxes of fewer lines (the edges above)
+    assert check(n, (1.0, 1.0, 1.0), 1e-8, 7) <= 3
