@@ -11,7 +11,10 @@
 namespace rb200 {
 
 constexpr int DCT_THREADS = 256;
-constexpr int DCT_KB = 16;  // table rows staged at a time
+// Table rows staged at a time, with a block barrier for each lot (us per solve,
+// 16 rows / 32: 256^3 1979 / 1872, 128^3 302 / 295, 512x64x64 413 / 392; 64 boxes
+// 2.55 / 2.45 ms of a step).
+constexpr int DCT_KB = 32;
 
 __host__ __device__ __forceinline__ int dct_row_pitch(int neP, int noP) { return ((neP + noP + 31) & ~31) + 4; }
 
@@ -141,9 +144,9 @@ __device__ __forceinline__ void dct_product(float (&ae)[RM][4], float (&ao)[RM][
 // moved, and the tables come from L2. A whole line set per block (a 64 KB tile
 // at n = 256) keeps the element traffic at one read and one write a pass; 8 x 4
 // outputs a thread take three 16-byte reads for 32 multiply-adds, issued two at
-// a time (paired: the six transforms of 256^3 920 us against 990 one at a time,
-// in a step 3436 against 3610). 8 x 8 outputs, three quarters of the reads but
-// half the warps, took 5% longer on a step of 256^3 and 7% on one of 128^3.
+// a time (paired: the five passes of 256^3 857 us against 936 one at a time, in
+// a step 3436 against 3610). 8 x 8 outputs, three quarters of the reads but half
+// the warps, took 5% longer on a step of 256^3 and 7% on one of 128^3.
 // The whole lines of the tile are staged in shared
 // memory before anything is written, so src and dst may be the same array.
 // `cold`: read src64 instead of src.
