@@ -476,6 +476,19 @@ __device__ __noinline__ bool sgs_poll(const unsigned long long* p, unsigned tag,
     }
 }
 
+// The slot of the step values (first buffer) that line q of an incoming face
+// fills: beside row q + 1 for the y face, above column q + 1 for the z face. A
+// face has as many slots as a unit has lines across it.
+__host__ __device__ constexpr int sgs_face_slots(bool z) { return z ? SGS_UJ : SGS_UK; }
+__host__ __device__ constexpr int sgs_face_slot(bool z, int q) { return z ? q + 1 : (q + 1) * SGS_VP; }
+constexpr bool sgs_face_slots_fit() {
+    for (int z = 0; z < 2; ++z)
+        for (int q = 0; q < sgs_face_slots(z != 0); ++q)
+            if (q >= 16 || sgs_face_slot(z != 0, q) >= SGS_VALS) return false;
+    return true;
+}
+static_assert(sgs_face_slots_fit(), "a face has at most 16 lanes, its slots lie inside one buffer of step values");
+
 // The incoming faces' warp of a unit: lane q fetches line q of the y face, lane
 // 16 + q of the z face, one step of the unit at a time. The words come through
 // asynchronous copies, since a load into registers would be waited for at the
@@ -491,8 +504,8 @@ __device__ __forceinline__ void sgs_faces(const GridDev& g, const SgsFlow& f, co
     const bool has = q < lines && (REV ? b + 1 < nb : b > 0);
     const int line = (zf ? U.j0 : U.k0) + (REV ? lines - 1 - q : q);
     const unsigned long long* base = words + (has ? sgs_word(g, f, zf, REV ? b : b - 1, line) : 0);
-    double* const to = vals + (zf ? q + 1 : (q + 1) * SGS_VP);
-    if (!has) to[0] = to[SGS_VALS] = -0.0;
+    double* const to = vals + sgs_face_slot(zf, q);
+    if (!has && q < sgs_face_slots(zf)) to[0] = to[SGS_VALS] = -0.0;
     if (!__any_sync(0xffffffffu, has)) {
         __syncthreads();
         for (int t = 0; t < steps; ++t) sgs_step_end(t, steps);
