@@ -11,13 +11,13 @@
 // corrected buffers and publishes by rotating buffer indices on the device.
 #include <cmath>
 #include <memory>
-#include <mutex>
 #include <new>
 #include <string>
 
 #include "advect.cuh"
 #include "internal.hpp"
 #include "carrier.hpp"
+#include "coop.hpp"
 #include "direct_device.cuh"
 #include "project.cuh"
 
@@ -560,19 +560,6 @@ int rb200_carrier_profile(rb200_carrier* carrier, int which, int launches, doubl
     return carrier->solver.profile(which, launches, avg_ms);
 }
 
-// Steps whose solve is the persistent (cooperative, grid-barrier) kernel are
-// ordered one after another on each device: two such kernels never compete
-// for co-residency. Other carriers' steps overlap freely.
-static cudaEvent_t cooperative_lane(int device) {
-    static std::mutex mu;
-    static cudaEvent_t lanes[64] = {};
-    if (device < 0 || device >= 64) return nullptr;
-    std::lock_guard<std::mutex> lock(mu);
-    if (!lanes[device] && cudaEventCreateWithFlags(&lanes[device], cudaEventDisableTiming) != cudaSuccess)
-        lanes[device] = nullptr;
-    return lanes[device];
-}
-
 static int launch_step(rb200_carrier* carrier, const rb200_step_params* params, int project_only);
 
 int rb200_carrier_step_async(rb200_carrier* carrier, const rb200_step_params* params) {
@@ -622,13 +609,14 @@ static int launch_step(rb200_carrier* carrier, const rb200_step_params* params, 
                                cudaMemcpyHostToDevice, c->stream));
     if (c->lq_d)
         RB200_CUDA(cudaMemcpyAsync(c->lflow_d, c->lflow_h, sizeof(LiquidFlowDev), cudaMemcpyHostToDevice, c->stream));
-    cudaEvent_t lane = c->solver.persistent_blocks() ? cooperative_lane(c->device) : nullptr;
-    if (c->solver.persistent_blocks() && !lane) return RB200_EXECUTION;
-    if (lane) RB200_CUDA(cudaStreamWaitEvent(c->stream, lane, 0));
+    // a step whose solve is a cooperative kernel takes its lanes; other steps overlap freely
+    CoopTurn turn;
+    int rc = turn.begin(c->stream, c->solver.persistent_blocks());
+    if (rc) return rc;
     RB200_CUDA(cudaEventRecord(c->ev[2], c->stream));
     RB200_CUDA(cudaGraphLaunch(c->step_exec, c->stream));
     RB200_CUDA(cudaEventRecord(c->ev[3], c->stream));
-    if (lane) RB200_CUDA(cudaEventRecord(lane, c->stream));
+    if ((rc = turn.end())) return rc;
     c->in_flight = true;
     return RB200_OK;
 }

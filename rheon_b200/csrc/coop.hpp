@@ -1,0 +1,37 @@
+// Admission of cooperative kernels to a device (coop.cu).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <mutex>
+
+namespace rb200 {
+
+// One launch (or graph launch) that holds a cooperative kernel:
+//
+//     CoopTurn turn;
+//     if ((rc = turn.begin(stream, blocks))) return rc;
+//     ... the launch on `stream` ...
+//     if ((rc = turn.end())) return rc;
+//
+// begin makes the stream wait for the launches whose lanes this one takes; end
+// records its own end on them. The device's lanes stay locked in between, so
+// that no other thread's launch comes between the wait and the record. Nothing
+// here waits on the host for the device. blocks = 0 (no cooperative kernel)
+// takes no lane.
+class CoopTurn {
+public:
+    CoopTurn() = default;
+    CoopTurn(const CoopTurn&) = delete;
+    CoopTurn& operator=(const CoopTurn&) = delete;
+    int begin(cudaStream_t s, int blocks);
+    int end();
+
+private:
+    std::unique_lock<std::mutex> lock_;
+    struct CoopDevice* dev_ = nullptr;
+    cudaStream_t stream_ = nullptr;
+    unsigned taken_ = 0;  // bit per lane
+};
+
+}  // namespace rb200
