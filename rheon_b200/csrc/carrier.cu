@@ -17,7 +17,6 @@
 #include "advect.cuh"
 #include "internal.hpp"
 #include "carrier.hpp"
-#include "coop.hpp"
 #include "direct_device.cuh"
 #include "project.cuh"
 
@@ -611,7 +610,7 @@ static int launch_step(rb200_carrier* carrier, const rb200_step_params* params, 
         RB200_CUDA(cudaMemcpyAsync(c->lflow_d, c->lflow_h, sizeof(LiquidFlowDev), cudaMemcpyHostToDevice, c->stream));
     // a step whose solve is a cooperative kernel takes its lanes; other steps overlap freely
     CoopTurn turn;
-    int rc = turn.begin(c->stream, c->solver.persistent_blocks());
+    int rc = turn.begin(c->stream, c->solver.persistent_blocks(), c->solver.user());
     if (rc) return rc;
     RB200_CUDA(cudaEventRecord(c->ev[2], c->stream));
     RB200_CUDA(cudaGraphLaunch(c->step_exec, c->stream));

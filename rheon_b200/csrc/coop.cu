@@ -18,6 +18,7 @@
 // per-pass kernels that the resident one replaced took 3.4, 6.3, 7.0 and 13.6.
 #include "coop.hpp"
 
+#include <atomic>
 #include <cstdint>
 
 #include "internal.hpp"
@@ -28,18 +29,25 @@ namespace {
 constexpr int kLanes = 4;
 }
 
+uint64_t coop_user() {
+    static std::atomic<uint64_t> last{0};
+    return ++last;
+}
+
 struct CoopDevice {
     std::mutex mu;
     int sms = 0;  // 0: not set up
     uint64_t turns = 0;
+    // the ends of the lanes' last launches: one event more than lanes, so that
+    // one is free for the next launch
+    cudaEvent_t done[kLanes + 1] = {};
     struct {
-        cudaEvent_t done = nullptr;  // the end of the last launch that took the lane
-        cudaStream_t last = nullptr;
-        uint64_t turn = 0;
+        int done = -1;  // -1: nothing to wait for
+        uint64_t user = 0, turn = 0;
     } lane[kLanes];
 };
 
-int CoopTurn::begin(cudaStream_t s, int blocks) {
+int CoopTurn::begin(cudaStream_t s, int blocks, uint64_t user) {
     if (blocks < 1) return RB200_OK;
     static CoopDevice devices[64];
     int id = 0;
@@ -51,31 +59,33 @@ int CoopTurn::begin(cudaStream_t s, int blocks) {
     CoopDevice& d = devices[id];
     lock_ = std::unique_lock<std::mutex>(d.mu);
     if (!d.sms) {
-        for (auto& l : d.lane)
-            if (!l.done) RB200_CUDA(cudaEventCreateWithFlags(&l.done, cudaEventDisableTiming));
+        for (auto& e : d.done)
+            if (!e) RB200_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         RB200_CUDA(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, id));
     }
     const int width = d.sms / kLanes;
     int want = kLanes;
     while (want > 1 && blocks <= (want - 1) * width) --want;
-    // the stream's own lanes first (no other launch is held up by them), then
-    // the ones taken longest ago
+    // the user's own lanes first (no other launch is held up by them), then the
+    // ones taken longest ago
     taken_ = 0;
+    unsigned waited = 0;  // bit per event
     for (int q = 0; q < want; ++q) {
         int best = -1;
         for (int l = 0; l < kLanes; ++l) {
             if (taken_ & (1u << l)) continue;
-            const bool own = d.lane[l].last == s;
-            if (best < 0 || own > (d.lane[best].last == s) ||
-                (own == (d.lane[best].last == s) && d.lane[l].turn < d.lane[best].turn))
-                best = l;
+            const bool own = d.lane[l].user == user, best_own = best >= 0 && d.lane[best].user == user;
+            if (best < 0 || own > best_own || (own == best_own && d.lane[l].turn < d.lane[best].turn)) best = l;
         }
         taken_ |= 1u << best;
-        // its own lane too: a stream's handle may come back for a new stream
-        RB200_CUDA(cudaStreamWaitEvent(s, d.lane[best].done, 0));
+        const auto& lane = d.lane[best];
+        if (lane.user == user || lane.done < 0 || (waited & (1u << lane.done))) continue;
+        waited |= 1u << lane.done;
+        RB200_CUDA(cudaStreamWaitEvent(s, d.done[lane.done], 0));
     }
     dev_ = &d;
     stream_ = s;
+    user_ = user;
     return RB200_OK;
 }
 
@@ -83,11 +93,17 @@ int CoopTurn::end() {
     if (!dev_) return RB200_OK;
     CoopDevice& d = *dev_;
     dev_ = nullptr;
+    unsigned used = 0;
+    for (int l = 0; l < kLanes; ++l)
+        if (!(taken_ & (1u << l)) && d.lane[l].done >= 0) used |= 1u << d.lane[l].done;
+    int event = 0;
+    while (used & (1u << event)) ++event;
+    RB200_CUDA(cudaEventRecord(d.done[event], stream_));
     ++d.turns;
     for (int l = 0; l < kLanes; ++l) {
         if (!(taken_ & (1u << l))) continue;
-        RB200_CUDA(cudaEventRecord(d.lane[l].done, stream_));
-        d.lane[l].last = stream_;
+        d.lane[l].done = event;
+        d.lane[l].user = user_;
         d.lane[l].turn = d.turns;
     }
     lock_.unlock();

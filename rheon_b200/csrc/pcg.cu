@@ -1433,7 +1433,12 @@ int PcgSolver::capture_chunk() {
 }
 
 int PcgSolver::launch_chunk(int slot) {
+    // a chunk that is a cooperative kernel takes its lanes, as a carrier's step does
+    CoopTurn turn;
+    int rc = turn.begin(stream_, persist_blocks_, user_);
+    if (rc) return rc;
     RB200_CUDA(cudaGraphLaunch(chunk_exec_, stream_));
+    if ((rc = turn.end())) return rc;
     launches_ += uint64_t(nodes_per_chunk_);
     return record_flags(slot);
 }
@@ -1657,6 +1662,9 @@ int PcgSolver::profile(int which, int launches, double* avg_ms) {
     if (which == 2) {
         // one warm iteration, then `launches` iterations in one launch
         RB200_CUDA(reset_persistent(stream_));
+        CoopTurn turn;
+        int rc = turn.begin(stream_, persist_blocks_, user_);
+        if (rc) return rc;
         RB200_CUDA(launch_persistent_chunk(stream_, 1, nullptr));
         cudaEvent_t a, b;
         RB200_CUDA(cudaEventCreate(&a));
@@ -1664,6 +1672,7 @@ int PcgSolver::profile(int which, int launches, double* avg_ms) {
         RB200_CUDA(cudaEventRecord(a, stream_));
         RB200_CUDA(launch_persistent_chunk(stream_, launches, nullptr));
         RB200_CUDA(cudaEventRecord(b, stream_));
+        if ((rc = turn.end())) return rc;
         RB200_CUDA(cudaEventSynchronize(b));
         float ms = 0.0f;
         cudaEventElapsedTime(&ms, a, b);

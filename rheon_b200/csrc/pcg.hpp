@@ -4,6 +4,7 @@
 
 #include <cuda.h>
 
+#include "coop.hpp"
 #include "direct.hpp"
 #include "internal.hpp"
 #include "mg.hpp"
@@ -137,6 +138,7 @@ public:
     int nodes_per_chunk() const { return nodes_per_chunk_ + 1; }
     // Blocks of the persistent solver kernel (0: the per-pass kernels run).
     int persistent_blocks() const { return persist_blocks_; }
+    uint64_t user() const { return user_; }  // of cooperative launches (coop.hpp)
     // One launch of the persistent kernel for at most `budget` iterations.
     cudaError_t launch_persistent_chunk(cudaStream_t s, int budget) { return launch_persistent_chunk(s, budget, d_trace_); }
     cudaError_t launch_persistent_chunk(cudaStream_t s, int budget, rb200_trace* trace);
@@ -189,6 +191,7 @@ private:
     SgsFlow sgs_{};
     double* ppart_ = nullptr;
     ResidentPlan resident_{};
+    const uint64_t user_ = coop_user();
     unsigned long long* rwords_ = nullptr;
 };
 
