@@ -9,6 +9,7 @@
 // accepted state is never written by a rejected step (transactional, as
 // commit_prepared, src/simulation.rs:805-811): the step writes candidate and
 // corrected buffers and publishes by rotating buffer indices on the device.
+#include <atomic>
 #include <cmath>
 #include <memory>
 #include <new>
@@ -251,6 +252,16 @@ int launch_validate_faces(const GridDev& g, const T* u, const T* v, const T* w, 
 
 }  // namespace rb200
 
+// Cooperative steps in flight on a device.
+static std::atomic<int>& cooperative_steps(int device) {
+    static std::atomic<int> steps[64] = {};
+    return steps[device & 63];
+}
+
+void rb200::cooperative_step_ended(const rb200_carrier& c) {
+    if (c.solver.persistent_blocks() > 0) --cooperative_steps(c.device);
+}
+
 using namespace rb200;
 
 namespace {
@@ -277,7 +288,7 @@ int blocks_for(long long n, int threads, int cap) {
 }
 
 template <class T>
-int capture_step(rb200_carrier* c) {
+int capture_step(rb200_carrier* c, cudaGraphExec_t* exec, bool beside) {
     const GridDev& g = c->g;
     cudaStream_t s = c->stream;
     const long long faces = (long long)g.flen[0] + g.flen[1] + g.flen[2];
@@ -304,7 +315,7 @@ int capture_step(rb200_carrier* c) {
         rc = c->accepted_p
                  ? c->solver.enqueue_reset(&c->cd->dt, &c->cd->skip, c->cfg.settings, s, &c->cd->warm, c->accepted_p)
                  : c->solver.enqueue_reset(&c->cd->dt, &c->cd->skip, c->cfg.settings, s);
-    if (!rc) rc = c->solver.enqueue_loop(s, c->body_stream, c->cfg.settings);
+    if (!rc) rc = c->solver.enqueue_loop(s, c->body_stream, c->cfg.settings, beside);
     if (rc) {
         cudaGraph_t dummy = nullptr;
         cudaStreamEndCapture(s, &dummy);
@@ -337,7 +348,7 @@ int capture_step(rb200_carrier* c) {
         set_error(std::string("step capture: ") + cudaGetErrorString(le != cudaSuccess ? le : ee));
         return RB200_EXECUTION;
     }
-    cudaError_t ie = cudaGraphInstantiate(&c->step_exec, graph, 0);
+    cudaError_t ie = cudaGraphInstantiate(exec, graph, 0);
     cudaGraphDestroy(graph);
     if (ie != cudaSuccess) {
         set_error(std::string("step graph instantiate: ") + cudaGetErrorString(ie));
@@ -347,6 +358,10 @@ int capture_step(rb200_carrier* c) {
     // (+ seed and keep kernels with the warm-start policy)
     c->fixed_nodes = 5 + (c->tracer[0] ? 1 : 0) + (c->accepted_p ? 2 : 0) + (c->lq_d ? 2 : 0);
     return RB200_OK;
+}
+
+int capture_step(rb200_carrier* c, cudaGraphExec_t* exec, bool beside) {
+    return c->elem == 4 ? capture_step<float>(c, exec, beside) : capture_step<double>(c, exec, beside);
 }
 
 int upload_rate(rb200_carrier* c) {
@@ -456,7 +471,7 @@ int rb200_carrier_create(const rb200_carrier_config* config, rb200_carrier** out
     if ((rc = c->solver.init(g, config->method, c->stream))) return rc;
     c->bytes += c->solver.bytes();
     RB200_CUDA(cudaStreamSynchronize(c->stream));
-    rc = c->elem == 4 ? capture_step<float>(c.get()) : capture_step<double>(c.get());
+    rc = capture_step(c.get(), &c->step_exec, false);
     if (rc) return rc;
     *out = c.release();
     return RB200_OK;
@@ -559,10 +574,10 @@ int rb200_carrier_profile(rb200_carrier* carrier, int which, int launches, doubl
     return carrier->solver.profile(which, launches, avg_ms);
 }
 
-static int launch_step(rb200_carrier* carrier, const rb200_step_params* params, int project_only);
+static int launch_step(rb200_carrier* carrier, const rb200_step_params* params, int project_only, bool together);
 
 int rb200_carrier_step_async(rb200_carrier* carrier, const rb200_step_params* params) {
-    return launch_step(carrier, params, 0);
+    return launch_step(carrier, params, 0, false);
 }
 
 // ProjectionStepWorkspace::project (src/projection_step.rs:863-1033) on the
@@ -575,7 +590,7 @@ int rb200_carrier_project_async(rb200_carrier* carrier, const rb200_step_params*
         carrier->err = "a projection takes its dt as requested and carries no tracer or liquid state";
         return RB200_INVALID_ARGUMENT;
     }
-    return launch_step(carrier, params, 1);
+    return launch_step(carrier, params, 1, false);
 }
 
 int rb200_carrier_project(rb200_carrier* carrier, const rb200_step_params* params, rb200_step_report* report) {
@@ -586,7 +601,8 @@ int rb200_carrier_project(rb200_carrier* carrier, const rb200_step_params* param
     return rb200_carrier_step_wait(carrier, report);
 }
 
-static int launch_step(rb200_carrier* carrier, const rb200_step_params* params, int project_only) {
+// together: other carriers' steps are launched with this one.
+static int launch_step(rb200_carrier* carrier, const rb200_step_params* params, int project_only, bool together) {
     if (!carrier || !params) return RB200_INVALID_ARGUMENT;
     rb200_carrier* c = carrier;
     if (c->in_flight) return RB200_INVALID_ARGUMENT;
@@ -608,14 +624,20 @@ static int launch_step(rb200_carrier* carrier, const rb200_step_params* params, 
                                cudaMemcpyHostToDevice, c->stream));
     if (c->lq_d)
         RB200_CUDA(cudaMemcpyAsync(c->lflow_d, c->lflow_h, sizeof(LiquidFlowDev), cudaMemcpyHostToDevice, c->stream));
-    // a step whose solve is a cooperative kernel takes its lanes; other steps overlap freely
+    // A step whose solve is a cooperative kernel takes its lanes; other steps
+    // overlap freely. Beside other cooperative steps it takes half of the lanes
+    // where it can.
+    const bool cooperative = c->solver.persistent_blocks() > 0;
+    bool beside = c->solver.has_beside() && (together || cooperative_steps(c->device) > 0);
+    if (beside && !c->beside_exec && capture_step(c, &c->beside_exec, true)) beside = false;
     CoopTurn turn;
-    int rc = turn.begin(c->stream, c->solver.persistent_blocks(), c->solver.user());
+    int rc = turn.begin(c->stream, c->solver.persistent_blocks(beside), c->solver.user());
     if (rc) return rc;
     RB200_CUDA(cudaEventRecord(c->ev[2], c->stream));
-    RB200_CUDA(cudaGraphLaunch(c->step_exec, c->stream));
+    RB200_CUDA(cudaGraphLaunch(beside ? c->beside_exec : c->step_exec, c->stream));
     RB200_CUDA(cudaEventRecord(c->ev[3], c->stream));
     if ((rc = turn.end())) return rc;
+    if (cooperative) ++cooperative_steps(c->device);
     c->in_flight = true;
     return RB200_OK;
 }
@@ -632,6 +654,7 @@ int rb200_carrier_step_wait(rb200_carrier* carrier, rb200_step_report* report) {
     if (!c->in_flight) return RB200_INVALID_ARGUMENT;
     cudaSetDevice(c->device);
     c->in_flight = false;
+    cooperative_step_ended(*c);
     RB200_CUDA(cudaStreamSynchronize(c->stream));
     const CarrierDev& h = *c->h_cd;
     *report = h.report;
@@ -689,8 +712,9 @@ int rb200_carrier_attach_liquid(rb200_carrier* carrier, double density, rb200_li
     RB200_CUDA(cudaStreamSynchronize(c->stream));
     // the step graph now holds the liquid interval
     if (c->step_exec) cudaGraphExecDestroy(c->step_exec);
-    c->step_exec = nullptr;
-    return capture_step<float>(c);
+    if (c->beside_exec) cudaGraphExecDestroy(c->beside_exec);
+    c->step_exec = c->beside_exec = nullptr;
+    return capture_step(c, &c->step_exec, false);
 }
 
 // LiquidStepInputs' inlet, source and volume settings (src/liquid_step.rs)
@@ -777,8 +801,10 @@ int rb200_carriers_step(rb200_carrier* const* carriers, size_t count, const rb20
                         rb200_step_report* reports, int* statuses) {
     if (!carriers || !params || !reports || !statuses) return RB200_INVALID_ARGUMENT;
     int first_error = RB200_OK;
+    size_t cooperative = 0;
+    for (size_t i = 0; i < count; ++i) cooperative += carriers[i] && carriers[i]->solver.persistent_blocks() > 0;
     for (size_t i = 0; i < count; ++i) {
-        statuses[i] = rb200_carrier_step_async(carriers[i], &params[i]);
+        statuses[i] = launch_step(carriers[i], &params[i], 0, cooperative > 1);
         if (statuses[i] && !first_error) first_error = statuses[i];
     }
     for (size_t i = 0; i < count; ++i) {

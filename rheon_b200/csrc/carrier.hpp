@@ -10,6 +10,8 @@
 #include "liquid.hpp"
 #include "pcg.hpp"
 
+struct rb200_carrier;
+
 namespace rb200 {
 
 constexpr int STEP_RUNNING = -1;
@@ -53,6 +55,9 @@ struct CarrierDev {
 struct ForcedScratch;
 void forced_scratch_free(ForcedScratch* scratch);
 
+// A carrier's launched step is no longer in flight.
+void cooperative_step_ended(const rb200_carrier& carrier);
+
 }  // namespace rb200
 
 // Host side of the carrier (opaque handle of include/rheon_b200.h).
@@ -71,6 +76,7 @@ struct rb200_carrier {
     rb200::CarrierDev* h_cd = nullptr;    // pinned host mirror
     cudaEvent_t ev[4] = {};
     cudaGraphExec_t step_exec = nullptr;
+    cudaGraphExec_t beside_exec = nullptr;  // the step beside other cooperative ones, captured when first needed
     int fixed_nodes = 0;
     size_t bytes = 0;
     bool in_flight = false;
@@ -93,6 +99,8 @@ struct rb200_carrier {
         if (stream) cudaStreamSynchronize(stream);
         rb200::forced_scratch_free(forced);
         if (step_exec) cudaGraphExecDestroy(step_exec);
+        if (beside_exec) cudaGraphExecDestroy(beside_exec);
+        if (in_flight) rb200::cooperative_step_ended(*this);
         for (auto& b : faces)
             for (auto& a : b) cudaFree(a);
         cudaFree(tracer[0]);

@@ -25,10 +25,6 @@
 
 namespace rb200 {
 
-namespace {
-constexpr int kLanes = 4;
-}
-
 uint64_t coop_user() {
     static std::atomic<uint64_t> last{0};
     return ++last;
@@ -40,11 +36,11 @@ struct CoopDevice {
     uint64_t turns = 0;
     // the ends of the lanes' last launches: one event more than lanes, so that
     // one is free for the next launch
-    cudaEvent_t done[kLanes + 1] = {};
+    cudaEvent_t done[kCoopLanes + 1] = {};
     struct {
         int done = -1;  // -1: nothing to wait for
         uint64_t user = 0, turn = 0;
-    } lane[kLanes];
+    } lane[kCoopLanes];
 };
 
 int CoopTurn::begin(cudaStream_t s, int blocks, uint64_t user) {
@@ -63,8 +59,8 @@ int CoopTurn::begin(cudaStream_t s, int blocks, uint64_t user) {
             if (!e) RB200_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         RB200_CUDA(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, id));
     }
-    const int width = d.sms / kLanes;
-    int want = kLanes;
+    const int width = d.sms / kCoopLanes;
+    int want = kCoopLanes;
     while (want > 1 && blocks <= (want - 1) * width) --want;
     // the user's own lanes first (no other launch is held up by them), then the
     // ones taken longest ago
@@ -72,7 +68,7 @@ int CoopTurn::begin(cudaStream_t s, int blocks, uint64_t user) {
     unsigned waited = 0;  // bit per event
     for (int q = 0; q < want; ++q) {
         int best = -1;
-        for (int l = 0; l < kLanes; ++l) {
+        for (int l = 0; l < kCoopLanes; ++l) {
             if (taken_ & (1u << l)) continue;
             const bool own = d.lane[l].user == user, best_own = best >= 0 && d.lane[best].user == user;
             if (best < 0 || own > best_own || (own == best_own && d.lane[l].turn < d.lane[best].turn)) best = l;
@@ -94,13 +90,13 @@ int CoopTurn::end() {
     CoopDevice& d = *dev_;
     dev_ = nullptr;
     unsigned used = 0;
-    for (int l = 0; l < kLanes; ++l)
+    for (int l = 0; l < kCoopLanes; ++l)
         if (!(taken_ & (1u << l)) && d.lane[l].done >= 0) used |= 1u << d.lane[l].done;
     int event = 0;
     while (used & (1u << event)) ++event;
     RB200_CUDA(cudaEventRecord(d.done[event], stream_));
     ++d.turns;
-    for (int l = 0; l < kLanes; ++l) {
+    for (int l = 0; l < kCoopLanes; ++l) {
         if (!(taken_ & (1u << l))) continue;
         d.lane[l].done = event;
         d.lane[l].user = user_;

@@ -21,6 +21,8 @@ namespace rb200 {
 // here waits on the host for the device. blocks = 0 (no cooperative kernel)
 // takes no lane. `user` is the launching solver's number (coop_user); a solver
 // launches on one stream all its life, so its own launches need no wait.
+constexpr int kCoopLanes = 4;  // of a device's SMs
+
 uint64_t coop_user();  // a number that no other solver has
 
 class CoopTurn {

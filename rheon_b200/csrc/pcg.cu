@@ -1353,6 +1353,19 @@ int PcgSolver::init(const GridDev& g, int method, cudaStream_t stream) {
             resident_.q = 0;
         } else {
             chunk_ = 64;
+            // Carriers stepped together run two at a time where each takes two
+            // lanes (coop.cu), so where the plan takes more there is a second
+            // one, a longer run of cells a thread: slower alone (us per
+            // iteration 37^3 7.7 / 8.1, 45^3 8.1 / 8.4, 63^3 8.7 / 10.1, 75^3
+            // 14.4 / 23.1), faster two at a time (ms for eight carriers stepped
+            // together, one at a time / two: 37^3 20.1 / 10.7, 45^3 26.3 / 13.7,
+            // 63^3 39.8 / 23.2, 75^3 81 / 64, 95^3 102 / 91). Its blocks hold
+            // half the SMs or fewer, or there is none (above about 96^3).
+            int dev = 0, sms = 0;
+            RB200_CUDA(cudaGetDevice(&dev));
+            RB200_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+            const int half = (sms / kCoopLanes) * (kCoopLanes / 2);
+            if (resident_.blocks > half && (rc = resident_setup(g, &beside_, half))) return rc;
         }
     } else if ((method == RB200_JACOBI_PCG_V1 || method == RB200_RBSGS_PCG) && maps_.use && persist_allowed) {
         persist_pre_ = method == RB200_RBSGS_PCG ? 1 : 0;
@@ -1370,9 +1383,9 @@ int PcgSolver::init(const GridDev& g, int method, cudaStream_t stream) {
     return capture_chunk();
 }
 
-cudaError_t PcgSolver::launch_persistent_chunk(cudaStream_t s, int budget, rb200_trace* trace) {
+cudaError_t PcgSolver::launch_persistent_chunk(cudaStream_t s, int budget, rb200_trace* trace, bool beside) {
     if (resident_.q)
-        return launch_resident(resident_, g_, st_, b_, p_, r_, z_, d_[0], d_[1], rwords_, gbar_, trace, budget, s);
+        return launch_resident(beside ? beside_ : resident_, g_, st_, b_, p_, r_, z_, d_[0], d_[1], rwords_, gbar_, trace, budget, s);
     return launch_persistent(g_, st_, b_, p_, r_, z_, d_[0], d_[1], ppart_, gbar_, trace, maps_, persist_blocks_,
                              budget, s, persist_pre_);
 }
@@ -1542,7 +1555,7 @@ int PcgSolver::enqueue_reset_fused(const double* dt_dev, const int* skip, const 
     return RB200_OK;
 }
 
-int PcgSolver::enqueue_loop(cudaStream_t cs, cudaStream_t body_stream, const rb200_settings& settings) {
+int PcgSolver::enqueue_loop(cudaStream_t cs, cudaStream_t body_stream, const rb200_settings& settings, bool beside) {
     cudaStreamCaptureStatus status;
     cudaGraph_t graph = nullptr;
     const cudaGraphNode_t* deps = nullptr;
@@ -1567,7 +1580,7 @@ int PcgSolver::enqueue_loop(cudaStream_t cs, cudaStream_t body_stream, const rb2
     const Bufs B{b_, p_, r_, z_, d_[0], d_[1], r1_, st_, part_, d_trace_, maps_, sgs_, direct()};
     const Multigrid* mg = multigrid();
     if (persist_blocks_) {
-        RB200_CUDA(launch_persistent_chunk(body_stream, chunk_));
+        RB200_CUDA(launch_persistent_chunk(body_stream, chunk_, d_trace_, beside));
     } else if (mg) {
         // The multigrid restart (a whole V-cycle) as an IF node after the
         // true-residual check: its launches run only in trips that restart.

@@ -134,14 +134,17 @@ public:
     // rhs_init_body: only the state is reset here, the pass decides the start.
     bool fuses_rhs() const { return use_direct_; }
     int enqueue_reset_fused(const double* dt_dev, const int* skip, const rb200_settings& settings, cudaStream_t s);
-    int enqueue_loop(cudaStream_t capture_stream, cudaStream_t body_stream, const rb200_settings& settings);
+    // beside: with the launch plan that leaves half of the SMs to another solve.
+    int enqueue_loop(cudaStream_t capture_stream, cudaStream_t body_stream, const rb200_settings& settings,
+                     bool beside = false);
     int nodes_per_chunk() const { return nodes_per_chunk_ + 1; }
     // Blocks of the persistent solver kernel (0: the per-pass kernels run).
-    int persistent_blocks() const { return persist_blocks_; }
+    int persistent_blocks(bool beside = false) const { return beside ? beside_.blocks : persist_blocks_; }
+    bool has_beside() const { return beside_.q != 0; }
     uint64_t user() const { return user_; }  // of cooperative launches (coop.hpp)
     // One launch of the persistent kernel for at most `budget` iterations.
     cudaError_t launch_persistent_chunk(cudaStream_t s, int budget) { return launch_persistent_chunk(s, budget, d_trace_); }
-    cudaError_t launch_persistent_chunk(cudaStream_t s, int budget, rb200_trace* trace);
+    cudaError_t launch_persistent_chunk(cudaStream_t s, int budget, rb200_trace* trace, bool beside = false);
     // Zeroes the barrier (and the reduction words) before a solve.
     cudaError_t reset_persistent(cudaStream_t s);
     int persist_pre_ = 0;  // preconditioner of the persistent kernel: 0 Jacobi, 1 red-black SGS
@@ -191,6 +194,7 @@ private:
     SgsFlow sgs_{};
     double* ppart_ = nullptr;
     ResidentPlan resident_{};
+    ResidentPlan beside_{};  // the resident kernel on at most half of the SMs, where resident_ takes more
     const uint64_t user_ = coop_user();
     unsigned long long* rwords_ = nullptr;
 };

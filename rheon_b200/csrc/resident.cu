@@ -586,7 +586,7 @@ constexpr size_t kResidentSmemMax = 212 * 1024;  // beside the static arrays
 }  // namespace
 
 // ------------------------------------------------------------ host side
-int resident_setup(const GridDev& g, ResidentPlan* plan) {
+int resident_setup(const GridDev& g, ResidentPlan* plan, int blocks) {
     *plan = ResidentPlan{};
     int dev = 0, sms = 0, coop = 0;
     RB200_CUDA(cudaGetDevice(&dev));
@@ -594,6 +594,7 @@ int resident_setup(const GridDev& g, ResidentPlan* plan) {
     RB200_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     if (!coop) return RB200_OK;
     sms = std::min(sms, RMAXB);
+    if (blocks > 0) sms = std::min(sms, blocks);
     // the shortest run whose bricks all have an SM: the most SMs at work
     for (int q : {1, 2, 4, 8, 16, 32}) {
         const long long nbx = (g.n[0] + 31) / 32, nby = (g.n[1] + RY - 1) / RY, nbz = (g.n[2] + q - 1) / q;
