@@ -9,7 +9,6 @@
 // accepted state is never written by a rejected step (transactional, as
 // commit_prepared, src/simulation.rs:805-811): the step writes candidate and
 // corrected buffers and publishes by rotating buffer indices on the device.
-#include <atomic>
 #include <cmath>
 #include <memory>
 #include <new>
@@ -252,14 +251,8 @@ int launch_validate_faces(const GridDev& g, const T* u, const T* v, const T* w, 
 
 }  // namespace rb200
 
-// Cooperative steps in flight on a device.
-static std::atomic<int>& cooperative_steps(int device) {
-    static std::atomic<int> steps[64] = {};
-    return steps[device & 63];
-}
-
 void rb200::cooperative_step_ended(const rb200_carrier& c) {
-    if (c.solver.persistent_blocks() > 0) --cooperative_steps(c.device);
+    if (c.solver.persistent_blocks() > 0) --rb200::coop_active(c.device);
 }
 
 using namespace rb200;
@@ -628,7 +621,7 @@ static int launch_step(rb200_carrier* carrier, const rb200_step_params* params, 
     // overlap freely. Beside other cooperative steps it takes half of the lanes
     // where it can.
     const bool cooperative = c->solver.persistent_blocks() > 0;
-    bool beside = c->solver.has_beside() && (together || cooperative_steps(c->device) > 0);
+    bool beside = c->solver.has_beside() && (together || coop_active(c->device) > 0);
     if (beside && !c->beside_exec && capture_step(c, &c->beside_exec, true)) beside = false;
     CoopTurn turn;
     int rc = turn.begin(c->stream, c->solver.persistent_blocks(beside), c->solver.user());
@@ -637,7 +630,7 @@ static int launch_step(rb200_carrier* carrier, const rb200_step_params* params, 
     RB200_CUDA(cudaGraphLaunch(beside ? c->beside_exec : c->step_exec, c->stream));
     RB200_CUDA(cudaEventRecord(c->ev[3], c->stream));
     if ((rc = turn.end())) return rc;
-    if (cooperative) ++cooperative_steps(c->device);
+    if (cooperative) ++coop_active(c->device);
     c->in_flight = true;
     return RB200_OK;
 }

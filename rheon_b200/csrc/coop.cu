@@ -18,9 +18,6 @@
 // per-pass kernels that the resident one replaced took 3.4, 6.3, 7.0 and 13.6.
 #include "coop.hpp"
 
-#include <atomic>
-#include <cstdint>
-
 #include "internal.hpp"
 
 namespace rb200 {
@@ -28,6 +25,11 @@ namespace rb200 {
 uint64_t coop_user() {
     static std::atomic<uint64_t> last{0};
     return ++last;
+}
+
+std::atomic<int>& coop_active(int device) {
+    static std::atomic<int> active[64] = {};
+    return active[device & 63];
 }
 
 struct CoopDevice {

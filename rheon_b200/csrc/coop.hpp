@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <mutex>
 
@@ -24,6 +25,8 @@ namespace rb200 {
 constexpr int kCoopLanes = 4;  // of a device's SMs
 
 uint64_t coop_user();  // a number that no other solver has
+// Cooperative solves in flight on a device: carriers' steps and host-driven solves.
+std::atomic<int>& coop_active(int device);
 
 class CoopTurn {
 public:

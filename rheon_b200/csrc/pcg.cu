@@ -1175,6 +1175,7 @@ static void fill_report(const SolveState& f, rb200_report* report) {
 
 PcgSolver::~PcgSolver() {
     if (chunk_exec_) cudaGraphExecDestroy(chunk_exec_);
+    if (beside_chunk_exec_) cudaGraphExecDestroy(beside_chunk_exec_);
     for (auto& e : ev_)
         if (e) cudaEventDestroy(e);
     cudaFree(b_);
@@ -1292,6 +1293,7 @@ int PcgSolver::init(const GridDev& g, int method, cudaStream_t stream) {
     g_ = g;
     method_ = method;
     stream_ = stream;
+    RB200_CUDA(cudaGetDevice(&device_));
     if (method < RB200_JACOBI_PCG_V1 || method > RB200_MG_MIXED) return RB200_UNSUPPORTED;
     int rc = set_smem_attrs();
     if (rc) return rc;
@@ -1361,9 +1363,8 @@ int PcgSolver::init(const GridDev& g, int method, cudaStream_t stream) {
             // together, one at a time / two: 37^3 20.1 / 10.7, 45^3 26.3 / 13.7,
             // 63^3 39.8 / 23.2, 75^3 81 / 64, 95^3 102 / 91). Its blocks hold
             // half the SMs or fewer, or there is none (above about 96^3).
-            int dev = 0, sms = 0;
-            RB200_CUDA(cudaGetDevice(&dev));
-            RB200_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+            int sms = 0;
+            RB200_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
             const int half = (sms / kCoopLanes) * (kCoopLanes / 2);
             if (resident_.blocks > half && (rc = resident_setup(g, &beside_, half))) return rc;
         }
@@ -1380,7 +1381,7 @@ int PcgSolver::init(const GridDev& g, int method, cudaStream_t stream) {
             else chunk_ = 64;
         }
     }
-    return capture_chunk();
+    return capture_chunk(&chunk_exec_, false);
 }
 
 cudaError_t PcgSolver::launch_persistent_chunk(cudaStream_t s, int budget, rb200_trace* trace, bool beside) {
@@ -1405,15 +1406,16 @@ int PcgSolver::set_trace(rb200_trace* host, size_t capacity) {
     h_trace_ = host;
     trace_cap_ = host ? capacity : 0;
     if (trace_cap_) RB200_CUDA(cudaMalloc(&d_trace_, trace_cap_ * sizeof(rb200_trace)));
-    if (chunk_exec_) {
-        cudaGraphExecDestroy(chunk_exec_);
-        chunk_exec_ = nullptr;
-    }
-    return capture_chunk();
+    for (cudaGraphExec_t* exec : {&chunk_exec_, &beside_chunk_exec_})
+        if (*exec) {
+            cudaGraphExecDestroy(*exec);
+            *exec = nullptr;
+        }
+    return capture_chunk(&chunk_exec_, false);
 }
 
 // One chunk: `chunk_` iterations, then the gated true-residual and restart.
-int PcgSolver::capture_chunk() {
+int PcgSolver::capture_chunk(cudaGraphExec_t* exec, bool beside) {
     const Bufs B{b_, p_, r_, z_, d_[0], d_[1], r1_, st_, part_, d_trace_, maps_, sgs_, direct()};
     const Multigrid* mg = multigrid();
     cudaGraph_t graph = nullptr;
@@ -1421,7 +1423,7 @@ int PcgSolver::capture_chunk() {
     int nodes = 0;
     cudaError_t launch_err = cudaSuccess;
     if (persist_blocks_) {
-        launch_err = launch_persistent_chunk(stream_, chunk_);
+        launch_err = launch_persistent_chunk(stream_, chunk_, d_trace_, beside);
         nodes = 1;
     } else {
         for (int q = 0; q < chunk_; ++q) nodes += launch_iteration(g_, method_, B, mg, stream_);
@@ -1436,7 +1438,7 @@ int PcgSolver::capture_chunk() {
                   cudaGetErrorString(launch_err != cudaSuccess ? launch_err : end_err));
         return RB200_EXECUTION;
     }
-    cudaError_t e = cudaGraphInstantiate(&chunk_exec_, graph, 0);
+    cudaError_t e = cudaGraphInstantiate(exec, graph, 0);
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) {
         set_error(std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
@@ -1448,9 +1450,9 @@ int PcgSolver::capture_chunk() {
 int PcgSolver::launch_chunk(int slot) {
     // a chunk that is a cooperative kernel takes its lanes, as a carrier's step does
     CoopTurn turn;
-    int rc = turn.begin(stream_, persist_blocks_, user_);
+    int rc = turn.begin(stream_, persistent_blocks(beside_now_), user_);
     if (rc) return rc;
-    RB200_CUDA(cudaGraphLaunch(chunk_exec_, stream_));
+    RB200_CUDA(cudaGraphLaunch(beside_now_ ? beside_chunk_exec_ : chunk_exec_, stream_));
     if ((rc = turn.end())) return rc;
     launches_ += uint64_t(nodes_per_chunk_);
     return record_flags(slot);
@@ -1480,6 +1482,16 @@ int PcgSolver::solve(double dt, const rb200_settings& s, rb200_report* report, r
     if (d_trace_) RB200_CUDA(cudaMemsetAsync(d_trace_, 0, trace_cap_ * sizeof(rb200_trace), stream_));
     RB200_CUDA(cudaMemsetAsync(part_.ticket, 0, sizeof(unsigned), stream_));
     if (persist_blocks_) RB200_CUDA(reset_persistent(stream_));
+    // in flight until this function returns
+    struct Active {
+        std::atomic<int>* n;
+        explicit Active(std::atomic<int>* count) : n(count) {
+            if (n) ++*n;
+        }
+        ~Active() {
+            if (n) --*n;
+        }
+    } active(persist_blocks_ ? &coop_active(device_) : nullptr);
     launches_ += uint64_t(launch_start(g_, method_, Bufs{b_, p_, r_, z_, d_[0], d_[1], r1_, st_, part_, d_trace_, maps_, sgs_, direct()},
                                        multigrid(), stream_));
     if (use_direct_ && initial) launches_ += uint64_t(direct_.enqueue_seed(g_, st_, b_, p_, d_[0], part_, stream_));
@@ -1489,9 +1501,16 @@ int PcgSolver::solve(double dt, const rb200_settings& s, rb200_report* report, r
     RB200_CUDA(cudaStreamSynchronize(stream_));
     int rc;
     if ((rc = record_flags(0))) return rc;
-    // A chunk ahead of the flags keeps the device busy through long solves; the
-    // direct method's usual solve is one chunk, so it launches none ahead.
-    const bool ahead = !use_direct_;
+    // A chunk ahead of the flags keeps the device busy through long solves. The
+    // direct method's usual solve is one chunk, so it launches none ahead. Nor
+    // does a cooperative solve beside others, which keep the device busy: the
+    // last chunk would wait for their turns to do nothing.
+    const bool others = persist_blocks_ && coop_active(device_) > 1;
+    const bool ahead = !use_direct_ && !others;
+    // Beside others the solve takes half of the lanes where it can, from its first
+    // chunk to its last: a launch leaves z on the surfaces of its bricks only.
+    beside_now_ = others && has_beside();
+    if (beside_now_ && !beside_chunk_exec_ && capture_chunk(&beside_chunk_exec_, true)) beside_now_ = false;
     if (ahead && (rc = launch_chunk(1))) return rc;
     int slot = 0, last_it = -1, stalls = 0;
     bool cancelled_now = false;

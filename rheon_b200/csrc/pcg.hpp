@@ -156,7 +156,7 @@ public:
     uint64_t launches() const { return launches_; }
 
 private:
-    int capture_chunk();
+    int capture_chunk(cudaGraphExec_t* exec, bool beside);
     int sgs_setup();
     int launch_chunk(int slot);
     int record_flags(int slot);
@@ -182,6 +182,7 @@ private:
     SolveState* h_st_ = nullptr;  // pinned, one slot per in-flight chunk
     cudaEvent_t ev_[2] = {nullptr, nullptr};
     cudaGraphExec_t chunk_exec_ = nullptr;
+    cudaGraphExec_t beside_chunk_exec_ = nullptr;  // with beside_, captured when first needed
     int chunk_ = 16;
     rb200_trace* d_trace_ = nullptr;
     rb200_trace* h_trace_ = nullptr;
@@ -193,8 +194,10 @@ private:
     GridBarrier* gbar_ = nullptr;
     SgsFlow sgs_{};
     double* ppart_ = nullptr;
+    int device_ = 0;
     ResidentPlan resident_{};
     ResidentPlan beside_{};  // the resident kernel on at most half of the SMs, where resident_ takes more
+    bool beside_now_ = false;  // the host-driven solve in progress uses beside_
     const uint64_t user_ = coop_user();
     unsigned long long* rwords_ = nullptr;
 };
