@@ -1197,14 +1197,15 @@ PcgSolver::~PcgSolver() {
     if (h_st_) cudaFreeHost(h_st_);
 }
 
-// Whether a cooperative launch of the persistent kernel can sit in a CUDA
-// graph, inside the body of a WHILE conditional node (the resident carrier's
-// form). Checked once per process by capturing and instantiating such a graph
-// (nothing is launched).
-static bool persistent_graphs_supported(PcgSolver& solver) {
-    static std::once_flag once;
-    static bool supported = false;
-    std::call_once(once, [&] {
+// Whether a cooperative launch of the solver's kernel can sit in a CUDA graph,
+// inside the body of a WHILE conditional node (the resident carrier's form).
+// Checked once per process for the resident kernel and once for the streaming
+// ones, by capturing and instantiating such a graph (nothing is launched).
+static bool persistent_graphs_supported(PcgSolver& solver, bool resident) {
+    static std::once_flag onces[2];
+    static bool answers[2] = {false, false};
+    bool& supported = answers[resident];
+    std::call_once(onces[resident], [&] {
         cudaStream_t outer = nullptr, body_stream = nullptr;
         if (cudaStreamCreateWithFlags(&outer, cudaStreamNonBlocking) != cudaSuccess) return;
         if (cudaStreamCreateWithFlags(&body_stream, cudaStreamNonBlocking) != cudaSuccess) {
@@ -1233,11 +1234,9 @@ static bool persistent_graphs_supported(PcgSolver& solver) {
                 ok = cudaStreamBeginCaptureToGraph(body_stream, body, nullptr, nullptr, 0,
                                                    cudaStreamCaptureModeRelaxed) == cudaSuccess;
                 if (ok) {
-                    const GridDev& gd = solver.grid();
                     cudaError_t le = solver.launch_persistent_chunk(body_stream, 1);
                     cudaGraph_t captured = nullptr;
                     cudaError_t ee = cudaStreamEndCapture(body_stream, &captured);
-                    (void)gd;
                     ok = le == cudaSuccess && ee == cudaSuccess;
                 }
                 ok = ok && cudaStreamUpdateCaptureDependencies(outer, &node, 1, cudaStreamSetCaptureDependencies) ==
@@ -1350,7 +1349,7 @@ int PcgSolver::init(const GridDev& g, int method, cudaStream_t stream) {
         bytes_ += words * sizeof(unsigned long long);
         RB200_CUDA(reset_persistent(stream_));
         persist_blocks_ = resident_.blocks;
-        if (!persistent_graphs_supported(*this)) {
+        if (!persistent_graphs_supported(*this, true)) {
             persist_blocks_ = 0;
             resident_.q = 0;
         } else {
@@ -1377,7 +1376,7 @@ int PcgSolver::init(const GridDev& g, int method, cudaStream_t stream) {
             RB200_CUDA(cudaMemsetAsync(gbar_, 0, sizeof(GridBarrier), stream_));
             if ((rc = alloc(&ppart_, persistent_partial_doubles(blocks)))) return rc;
             persist_blocks_ = blocks;
-            if (!persistent_graphs_supported(*this)) persist_blocks_ = 0;
+            if (!persistent_graphs_supported(*this, false)) persist_blocks_ = 0;
             else chunk_ = 64;
         }
     }
