@@ -1037,13 +1037,17 @@ static bool encode_box_map(CUtensorMap* m, const double* base, const GridDev& g)
     return encode_map(m, base, g, box);
 }
 
+// The maps of a solver's vectors. The encoder takes a null address, and a load
+// through such a map reads address 0: a solver without z or a second direction
+// (the direct method) has no maps, and without r (its timing run) no map of r,
+// which the direction pass does not read.
 static TmaMaps make_maps(const GridDev& g, const double* z, const double* d0, const double* d1, const double* p,
                          const double* r) {
     TmaMaps m;
     std::memset(&m, 0, sizeof(m));
-    if (tma_eligible(g) && encode_slab_map(&m.z, z, g) && encode_slab_map(&m.d0, d0, g) &&
+    if (z && d0 && d1 && p && tma_eligible(g) && encode_slab_map(&m.z, z, g) && encode_slab_map(&m.d0, d0, g) &&
         encode_slab_map(&m.d1, d1, g) && encode_slab_map(&m.p, p, g) && encode_box_map(&m.p_box, p, g) &&
-        encode_box_map(&m.r_box, r, g))
+        (!r || encode_box_map(&m.r_box, r, g)))
         m.use = 1;
     else
         std::memset(&m, 0, sizeof(m));
@@ -1690,6 +1694,7 @@ int PcgSolver::profile(int which, int launches, double* avg_ms) {
             }
             RB200_CUDA(cudaMemsetAsync(*v, 0, size_t(g_.cells) * sizeof(double), stream_));
         }
+    const TmaMaps maps = use_direct_ ? make_maps(g_, z_, d_[0], d_[1], p_, r_) : maps_;
     if (which == 2) {
         // one warm iteration, then `launches` iterations in one launch
         RB200_CUDA(reset_persistent(stream_));
@@ -1720,15 +1725,15 @@ int PcgSolver::profile(int which, int launches, double* avg_ms) {
     }
     auto launch = [&]() {
         if (which == 0)
-            k_pass1<ZC><<<grid, block, kSmemPass1, stream_>>>(g_, st_, z_, d_[0], d_[1], nullptr, maps_, part_, nullptr);
+            k_pass1<ZC><<<grid, block, kSmemPass1, stream_>>>(g_, st_, z_, d_[0], d_[1], nullptr, maps, part_, nullptr);
         else if (jac)
-            k_pass2<ZC, 0><<<grid, block, kSmemSlab, stream_>>>(g_, st_, p_, r_, z_, d_[0], d_[1], maps_, part_,
+            k_pass2<ZC, 0><<<grid, block, kSmemSlab, stream_>>>(g_, st_, p_, r_, z_, d_[0], d_[1], maps, part_,
                                                                    nullptr);
         else if (method_ == RB200_SGS_PCG_V1)
-            k_pass2<ZC, 2><<<grid, block, kSmemSlab, stream_>>>(g_, st_, p_, r_, z_, d_[0], d_[1], maps_, part_,
+            k_pass2<ZC, 2><<<grid, block, kSmemSlab, stream_>>>(g_, st_, p_, r_, z_, d_[0], d_[1], maps, part_,
                                                                    nullptr);
         else
-            k_pass2<ZC, 1><<<grid, block, kSmemSlab, stream_>>>(g_, st_, p_, r_, z_, d_[0], d_[1], maps_, part_,
+            k_pass2<ZC, 1><<<grid, block, kSmemSlab, stream_>>>(g_, st_, p_, r_, z_, d_[0], d_[1], maps, part_,
                                                                     nullptr);
     };
     launch();  // warm
