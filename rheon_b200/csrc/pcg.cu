@@ -1685,13 +1685,25 @@ int PcgSolver::profile(int which, int launches, double* avg_ms) {
     RB200_CUDA(cudaMemcpyAsync(st_, &h_st_[0], sizeof(SolveState), cudaMemcpyHostToDevice, stream_));
     const bool jac = method_ == RB200_JACOBI_PCG_V1;
     const dim3 grid = slab_grid(g_), block(TX, TY, 1);
-    // the direct method keeps no z and no second direction for the timed pass
+    // the direct method keeps no z and no second direction: the timed pass gets
+    // some for this call
+    struct Lent {
+        double** v = nullptr;
+        ~Lent() {
+            if (!v) return;
+            cudaFree(*v);
+            *v = nullptr;
+        }
+    } lent[2];
+    int lends = 0;
     for (double** v : {&z_, &d_[1]})
         if (!*v) {
             if (cudaMalloc(v, size_t(g_.cells) * sizeof(double)) != cudaSuccess) {
                 cudaGetLastError();
+                *v = nullptr;
                 return RB200_OUT_OF_MEMORY;
             }
+            lent[lends++].v = v;
             RB200_CUDA(cudaMemsetAsync(*v, 0, size_t(g_.cells) * sizeof(double), stream_));
         }
     const TmaMaps maps = use_direct_ ? make_maps(g_, z_, d_[0], d_[1], p_, r_) : maps_;
