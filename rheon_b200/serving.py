@@ -113,12 +113,19 @@ def merge_completions(per_rank: Sequence[Sequence[Completion]]) -> List[Completi
 
 
 def carrier_bytes_estimate(edge: int, config: CarrierConfig) -> int:
-    """Device bytes of one carrier (three face buffers, solver vectors, the
-    FP32 preconditioner's), before it is created."""
+    """Device bytes of one carrier (three face buffers, the solver's vectors
+    and its preconditioner's), before it is created."""
     n = edge ** 3
     faces = 3 * edge * edge * (edge + 1)
     elem = 4 if config.storage == "f32" else 8
-    per_cell = 8 * 7 + (6 if config.implementation == 3 else 0) + (8 if config.warm_start else 0)
+    warm = 8 if config.warm_start else 0
+    mixed = config.implementation == 3
+    if mixed and 8 < edge <= 512:
+        # the direct solve: b and two iterates in f64, r and z in f32, and its
+        # tables of a quarter of edge^2 floats each, four of them
+        per_cell = 8 * 3 + 4 * 2 + (8 if config.with_tracer else 0) + warm
+        return 3 * faces * elem + n * per_cell + 4 * (edge + 32) ** 2 + (1 << 20)
+    per_cell = 8 * 7 + (6 if mixed else 0) + warm
     return 3 * faces * elem + n * per_cell + (1 << 20)
 
 
