@@ -286,7 +286,8 @@ __global__ void __launch_bounds__(DCT_THREADS, 2) k_b_dct(const BatchDctJob* __r
     if (st->flags & F_DONE) return;
     block_copy(J, job.J);
     __syncthreads();
-    dct_tile_any<ROW, OP>(J, sp.block, J.src64 != nullptr && st->it == 0, reinterpret_cast<float*>(dct_smem));
+    const float scale = ROW ? (OP == DCT_FORWARD ? st->down : st->up) : 1.0f;
+    dct_tile_any<ROW, OP>(J, sp.block, J.src64 != nullptr && st->it == 0, scale, reinterpret_cast<float*>(dct_smem));
 }
 
 // The right-hand side and the solve's start of the direct instances.

@@ -149,9 +149,10 @@ __device__ __forceinline__ void dct_product(float (&ae)[RM][4], float (&ao)[RM][
 // the warps, took 5% longer on a step of 256^3 and 7% on one of 128^3.
 // The whole lines of the tile are staged in shared
 // memory before anything is written, so src and dst may be the same array.
-// `cold`: read src64 instead of src.
+// `cold`: read src64 instead of src. `scale`: of what the first pass (ROW forward)
+// reads and of what the last one (ROW inverse) writes.
 template <int RM, bool ROW, int OP>
-__device__ __forceinline__ void dct_tile(const DctJob& J, int tile, bool cold, float* smem) {
+__device__ __forceinline__ void dct_tile(const DctJob& J, int tile, bool cold, float scale, float* smem) {
     const DctAxis& A = J.A;
     const int n = A.n, ne = A.ne, no = A.no, neP = A.neP, noP = A.noP;
     const int TC = 32 * J.nb, inner = J.inner;
@@ -185,11 +186,12 @@ __device__ __forceinline__ void dct_tile(const DctJob& J, int tile, bool cold, f
             if (cold) {
                 const double2 a = *reinterpret_cast<const double2*>(s64 + at);
                 const double2 b = *reinterpret_cast<const double2*>(s64 + at + 2);
-                return make_float4(float(a.x), float(a.y), float(b.x), float(b.y));
+                return make_float4(float(a.x) * scale, float(a.y) * scale, float(b.x) * scale, float(b.y) * scale);
             }
-            return *reinterpret_cast<const float4*>(src + at);
+            const float4 v = *reinterpret_cast<const float4*>(src + at);
+            return make_float4(v.x * scale, v.y * scale, v.z * scale, v.w * scale);
         };
-        auto ld1 = [&](int at) -> float { return cold ? float(s64[at]) : src[at]; };
+        auto ld1 = [&](int at) -> float { return (cold ? float(s64[at]) : src[at]) * scale; };
         if (vec && OP == DCT_FORWARD) {
             const int iq = ne >> 2;
 #pragma unroll 4
@@ -333,10 +335,10 @@ __device__ __forceinline__ void dct_tile(const DctJob& J, int tile, bool cold, f
                         if (m < ne) row[m] = ae[r][j];
                         if (m < no) row[ne + m] = ao[r][j];
                     } else if (m < no) {
-                        row[m] = ae[r][j] + ao[r][j];
-                        row[n - 1 - m] = ae[r][j] - ao[r][j];
+                        row[m] = (ae[r][j] + ao[r][j]) * scale;
+                        row[n - 1 - m] = (ae[r][j] - ao[r][j]) * scale;
                     } else if (m < ne) {
-                        row[m] = ae[r][j];
+                        row[m] = ae[r][j] * scale;
                     }
                 }
             }
@@ -392,13 +394,13 @@ __device__ __forceinline__ void dct_tile(const DctJob& J, int tile, bool cold, f
 }
 
 template <bool ROW, int OP>
-__device__ __forceinline__ void dct_tile_any(const DctJob& J, int tile, bool cold, float* smem) {
+__device__ __forceinline__ void dct_tile_any(const DctJob& J, int tile, bool cold, float scale, float* smem) {
     if (J.A.RM == 8)
-        dct_tile<8, ROW, OP>(J, tile, cold, smem);
+        dct_tile<8, ROW, OP>(J, tile, cold, scale, smem);
     else if (J.A.RM == 6)
-        dct_tile<6, ROW, OP>(J, tile, cold, smem);
+        dct_tile<6, ROW, OP>(J, tile, cold, scale, smem);
     else
-        dct_tile<4, ROW, OP>(J, tile, cold, smem);
+        dct_tile<4, ROW, OP>(J, tile, cold, scale, smem);
 }
 
 // build_rhs (project.cuh) with the start of a cold solve on it (the sums of b,
@@ -503,6 +505,7 @@ __device__ __forceinline__ void decide_refined(SolveState* st, rb200_trace* trac
     const double div = maximum * st->dt / volume;
     const double l2 = sqrt(squared);
     st->recursive_l2 = l2;
+    set_transform_scale(st, maximum);
     if (trace && it >= 1) {
         rb200_trace& t = trace[it - 1];
         t.alpha = 1.0;  // p += z
@@ -514,6 +517,7 @@ __device__ __forceinline__ void decide_refined(SolveState* st, rb200_trace* trac
         breakdown(st, it, flags);
         return;
     }
+    const double before = st->true_max;
     st->true_l2 = l2;
     st->true_max = maximum;
     st->true_div = div;
@@ -521,6 +525,8 @@ __device__ __forceinline__ void decide_refined(SolveState* st, rb200_trace* trac
         finish(st, RB200_OK, flags);
     else if (it == st->max_it)
         finish(st, RB200_ITERATION_LIMIT, flags);
+    else if (!seed && maximum < 0x1p-126 && !(maximum < 0.5 * before))
+        breakdown(st, it, flags);  // what FP32 holds of the residual below its normal range has nothing more to give
     else
         st->flags = flags;
 }

@@ -13,6 +13,21 @@ namespace rb200 {
 
 constexpr double kEps = 2.220446049250313e-16;
 
+// The powers of two by which the direct method's transforms scale the residual
+// that they read and the correction that they write, from the residual's largest
+// value. Inside, sums are up to sqrt(N) larger than the residual and products
+// 1e-7 smaller, so a residual that FP32 just holds would leave its range on
+// either side. Scaling by a power of two changes no other bit.
+__device__ __forceinline__ void set_transform_scale(SolveState* st, double largest) {
+    int e = 0;
+    if (largest > 0.0 && !(largest >= 0x1p-64 && largest <= 0x1p64)) {
+        frexp(largest, &e);
+        e = min(126, max(-126, e));
+    }
+    st->down = ldexpf(1.0f, -e);
+    st->up = ldexpf(1.0f, e);
+}
+
 // The decision of the start (src/pressure.rs:603-650) from the sums of b, |b|
 // and b^2 and the maxima: |b|, a non-finite b, a non-finite seed. Thread 0.
 __device__ __forceinline__ void decide_init(const GridDev& g, SolveState* st, const dd (&s)[3], const double (&m)[3],
@@ -44,6 +59,7 @@ __device__ __forceinline__ void decide_init(const GridDev& g, SolveState* st, co
             return;
         }
     }
+    set_transform_scale(st, m[0]);
     double rhs_l2 = sqrt(sq);
     double threshold = fmax(st->absolute, st->relative * rhs_l2);
     if (!isfinite(rhs_l2) || !isfinite(threshold)) {
