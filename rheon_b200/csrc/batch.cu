@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(BT) k_b_true_residual(const BatchInstDev* __re
                                                         const __grid_constant__ BatchSpans spans) {
     pdl_wait();
     __shared__ GridDev g;
-    __shared__ BlockReduce<2, 1> red;
+    __shared__ BlockReduce<3, 1> red;
     Span sp;
     const BatchInstDev& I = inst[batch_entry(spans, sp)];
     load_geometry(g, I.g);
@@ -390,6 +390,7 @@ __global__ void __launch_bounds__(BT) k_b_true_residual(const BatchInstDev* __re
     const double* __restrict__ p = I.p;
     const int n0 = g.n[0], n1 = g.n[1], n2 = g.n[2], sy = n0, sz = n0 * n1;
     Neu acc;
+    double total = 0.0;
     double gauge_sq = 0.0;
     double mx[1] = {0.0};
     for (int c = sp.block * blockDim.x + threadIdx.x; c < g.cells; c += sp.blocks * blockDim.x) {
@@ -405,14 +406,18 @@ __global__ void __launch_bounds__(BT) k_b_true_residual(const BatchInstDev* __re
         const double t = b[c] - apply_row(g, i, j, k, v);
         spare[c] = t;
         acc.add(t * t);
+        total += t;
         if (c == 0) gauge_sq = t * t;
         mx[0] = fmax(mx[0], fabs(t));
     }
-    dd sums[2] = {acc.as_dd(), dd_add1(acc.as_dd(), -gauge_sq)};
-    block_reduce<2, 1>(red, sums, mx);
-    if (publish_and_check_last<2, 1>(I.part, sp.block, sp.blocks, sums, mx)) {
-        fold_partials<2, 1>(I.part, sp.blocks, red, sums, mx);
-        if (threadIdx.x == 0) decide_true(st, nullptr, dd_value(sums[0]), dd_value(sums[1]), mx[0], flags, g.volume);
+    dd sums[3] = {acc.as_dd(), dd_add1(acc.as_dd(), -gauge_sq), dd{total, 0.0}};
+    block_reduce<3, 1>(red, sums, mx);
+    if (publish_and_check_last<3, 1>(I.part, sp.block, sp.blocks, sums, mx)) {
+        fold_partials<3, 1>(I.part, sp.blocks, red, sums, mx);
+        if (threadIdx.x == 0) {
+            st->load_mean = dd_value(sums[2]) / g.cells;
+            decide_true(st, nullptr, dd_value(sums[0]), dd_value(sums[1]), mx[0], flags, g.volume);
+        }
     }
 }
 

@@ -1133,16 +1133,17 @@ __device__ __forceinline__ void pass1_body(const GridDev& g, const MgLevelDev& L
 __device__ __forceinline__ void update_first_body(const GridDev& g, const MgLevelDev& L, SolveState* st,
                                                   double* __restrict__ p, double* r0, double* r1, const double* d0,
                                                   const double* d1, Partials part, rb200_trace* trace, Span sp) {
-    __shared__ BlockReduce<1, 0> red;
+    __shared__ BlockReduce<2, 0> red;
     const int flags = st->flags;
     if (flags & F_STOP) return;
-    const double alpha = st->alpha;
+    const double alpha = st->alpha, mean = st->mean;
     const double* __restrict__ d = st->dsel ? d1 : d0;
     // r_old is kept: the new residual goes to the other buffer
     const int rsel = st->rsel;
     const double* __restrict__ r = rsel ? r1 : r0;
     double* __restrict__ r_out = rsel ? r0 : r1;
     Neu acc;
+    double total = 0.0;
     const Warps W = span_warps(sp);
     const int n0 = g.n[0], rows = g.n[1] * g.n[2];
     for (int rw = W.w0; rw < rows; rw += W.nw) {
@@ -1165,8 +1166,9 @@ __device__ __forceinline__ void update_first_body(const GridDev& g, const MgLeve
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     pv[e] = pv[e] + alpha * dv[e];
-                    rv[e] = rv[e] - alpha * qv[e];
+                    rv[e] = (rv[e] - mean) - alpha * qv[e];
                     acc.add(rv[e] * rv[e]);
+                    total += rv[e];
                     f4put(bq, e, float(rv[e]));
                 }
 #pragma unroll
@@ -1186,8 +1188,9 @@ __device__ __forceinline__ void update_first_body(const GridDev& g, const MgLeve
             for (int i = W.lane; i < n0; i += 32) {
                 const int c = base + i;
                 p[c] = p[c] + alpha * d[c];
-                const double rc = r[c] - alpha * kd_at(g, d, i, j, k, c);
+                const double rc = (r[c] - mean) - alpha * kd_at(g, d, i, j, k, c);
                 acc.add(rc * rc);
+                total += rc;
                 r_out[c] = rc;
                 const float b = float(rc);
                 L.b[c] = b;
@@ -1196,14 +1199,15 @@ __device__ __forceinline__ void update_first_body(const GridDev& g, const MgLeve
             }
         }
     }
-    dd sums[1] = {acc.as_dd()};
+    dd sums[2] = {acc.as_dd(), dd{total, 0.0}};
     double none[1];
-    block_reduce<1, 0>(red, sums, none);
-    if (publish_and_check_last<1, 0>(part, sp.block, sp.blocks, sums, none)) {
-        fold_partials<1, 0>(part, sp.blocks, red, sums, none);
+    block_reduce<2, 0>(red, sums, none);
+    if (publish_and_check_last<2, 0>(part, sp.block, sp.blocks, sums, none)) {
+        fold_partials<2, 0>(part, sp.blocks, red, sums, none);
         if (threadIdx.x == 0) {
             st->rsel = rsel ^ 1;
             if (flags & F_PROFILE) return;
+            st->mean = dd_value(sums[1]) / g.cells;
             const int it = st->it + 1;
             st->it = it;
             const double recursive_l2 = sqrt(dd_value(sums[0]));

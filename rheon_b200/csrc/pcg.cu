@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(TILE_THREADS) k_true_residual(GridDev g, Solve
                                                                 rb200_trace* trace) {
     using S = Slab<ZC>;
     extern __shared__ __align__(128) double smem[];
-    __shared__ BlockReduce<2, 1> red;
+    __shared__ BlockReduce<3, 1> red;
     __shared__ __align__(8) uint64_t bar;
     const int flags = st->flags;
     if (!(flags & F_NEED_TRUE)) return;
@@ -267,6 +267,7 @@ __global__ void __launch_bounds__(TILE_THREADS) k_true_residual(GridDev g, Solve
     stage_issue<ZC>(g, maps, &bar, smem, p, &maps.p, nullptr, nullptr, nullptr, x0, y0, k0);
     if (!stage_wait(maps, &bar, st)) return;
     Neu acc;
+    double total = 0.0;
     double gauge_sq = 0.0;  // t[0]^2 when this thread holds cell 0
     double mx[1] = {0.0};
     const int i = x0 + threadIdx.x, j = y0 + threadIdx.y;
@@ -280,17 +281,21 @@ __global__ void __launch_bounds__(TILE_THREADS) k_true_residual(GridDev g, Solve
             double t = b[c] - apply_row(g, i, j, k0 + q, v);
             spare[c] = t;
             acc.add(t * t);
+            total += t;
             if (c == 0) gauge_sq = t * t;
             mx[0] = fmax(mx[0], fabs(t));
         }
     }
-    // the second sum leaves out the gauge row: |t[1..]|^2
-    dd sums[2] = {acc.as_dd(), dd_add1(acc.as_dd(), -gauge_sq)};
-    block_reduce<2, 1>(red, sums, mx);
+    // the second sum leaves out the gauge row: |t[1..]|^2; the third is of t itself
+    dd sums[3] = {acc.as_dd(), dd_add1(acc.as_dd(), -gauge_sq), dd{total, 0.0}};
+    block_reduce<3, 1>(red, sums, mx);
     const int nb = nblocks3();
-    if (publish_and_check_last<2, 1>(part, block_id3(), nb, sums, mx)) {
-        fold_partials<2, 1>(part, nb, red, sums, mx);
-        if (tid3() == 0) decide_true(st, trace, dd_value(sums[0]), dd_value(sums[1]), mx[0], flags, g.volume);
+    if (publish_and_check_last<3, 1>(part, block_id3(), nb, sums, mx)) {
+        fold_partials<3, 1>(part, nb, red, sums, mx);
+        if (tid3() == 0) {
+            st->load_mean = dd_value(sums[2]) / g.cells;
+            decide_true(st, trace, dd_value(sums[0]), dd_value(sums[1]), mx[0], flags, g.volume);
+        }
     }
 }
 
@@ -309,29 +314,32 @@ __global__ void __launch_bounds__(EW) k_mg_update(GridDev g, SolveState* st, dou
                                                   double* __restrict__ r, double* __restrict__ r_old,
                                                   const double* d0, const double* d1, Partials part,
                                                   rb200_trace* trace) {
-    __shared__ BlockReduce<1, 0> red;
+    __shared__ BlockReduce<2, 0> red;
     const int flags = st->flags;
     if (flags & F_STOP) return;
-    const double alpha = st->alpha;
+    const double alpha = st->alpha, mean = st->mean;
     const double* __restrict__ d = st->dsel ? d1 : d0;
     Neu acc;
+    double total = 0.0;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < g.cells; c += gridDim.x * blockDim.x) {
         int i, j, k;
         cell_coords(g, c, i, j, k);
         p[c] = p[c] + alpha * d[c];
         const double ro = r[c];
-        double rc = ro - alpha * kd_at(g, d, i, j, k, c);
+        double rc = (ro - mean) - alpha * kd_at(g, d, i, j, k, c);
         r_old[c] = ro;
         r[c] = rc;
         acc.add(rc * rc);
+        total += rc;
     }
-    dd sums[1] = {acc.as_dd()};
+    dd sums[2] = {acc.as_dd(), dd{total, 0.0}};
     double none[1];
-    block_reduce<1, 0>(red, sums, none);
-    if (publish_and_check_last<1, 0>(part, blockIdx.x, gridDim.x, sums, none)) {
-        fold_partials<1, 0>(part, gridDim.x, red, sums, none);
+    block_reduce<2, 0>(red, sums, none);
+    if (publish_and_check_last<2, 0>(part, blockIdx.x, gridDim.x, sums, none)) {
+        fold_partials<2, 0>(part, gridDim.x, red, sums, none);
         if (threadIdx.x == 0) {
             if (flags & F_PROFILE) return;
+            st->mean = dd_value(sums[1]) / g.cells;
             int it = st->it + 1;
             st->it = it;
             double recursive_l2 = sqrt(dd_value(sums[0]));
@@ -1837,7 +1845,7 @@ constexpr int kStaticMaxCells = 32768;   // 32^3 cells
 constexpr int kStaticMaxBlocks = 2048;   // blocks of the widest pass of a solve
 // Doubles of one block's reduction partials in the widest stage of a solve:
 // k_init_sums publishes 3 double-double sums and 3 maxima (2 * 3 + 3); the
-// other stages publish fewer (true residual 5, pass 2 4, pass 1 and the
+// other stages publish fewer (true residual 7, pass 2 4, pass 1 and the
 // residual load 2).
 constexpr int kStaticSlotDoubles = 2 * 3 + 3;
 constexpr size_t kStaticStateDoubles = 64;

@@ -32,6 +32,9 @@ struct SolveState {
     int flexible;       // beta = z.(r - r_old) / rz_old (flexible CG) instead of rz'/rz
     int trips;          // loop-body passes of the graph-embedded solve
     int rsel;           // flexible method: which residual buffer holds r (the update writes the other)
+    // flexible method: the means that the next load of a residual (from b or the
+    // true residual) and the next update take out of it
+    double load_mean, mean;
     float down, up;     // direct method: powers of two around its transforms (down up = 1)
 };
 

@@ -60,6 +60,7 @@ __device__ __forceinline__ void decide_init(const GridDev& g, SolveState* st, co
         }
     }
     set_transform_scale(st, m[0]);
+    st->load_mean = sum / g.cells;
     double rhs_l2 = sqrt(sq);
     double threshold = fmax(st->absolute, st->relative * rhs_l2);
     if (!isfinite(rhs_l2) || !isfinite(threshold)) {
@@ -142,12 +143,16 @@ __device__ __forceinline__ void load_residual_body(const GridDev& g, SolveState*
     const double* src = mode == MODE_INIT ? b : (st->dsel ? d0 : d1);
     // the flexible method alternates two residual buffers; a loaded residual
     // is in the first (the buffer the V-cycle's first half-sweep reads)
-    if (KIND == KIND_MG && sp.block == 0 && threadIdx.x == 0) st->rsel = 0;
+    if (KIND == KIND_MG && sp.block == 0 && threadIdx.x == 0) {
+        st->rsel = 0;
+        st->mean = 0.0;
+    }
     // ... and keeps the gauge row's residual (mg.hpp); the others eliminate it
     const bool full = KIND == KIND_MG && st->flexible;
+    const double mean = full ? st->load_mean : 0.0;
     Neu acc;
     for (int c = sp.block * blockDim.x + threadIdx.x; c < g.cells; c += sp.blocks * blockDim.x) {
-        double rc = c == 0 && !full ? 0.0 : src[c];
+        double rc = full ? src[c] - mean : (c == 0 ? 0.0 : src[c]);
         r[c] = rc;
         if (c == 0) {
             if (z) z[0] = 0.0;  // the multigrid method forms z in its own kernels and passes none
