@@ -794,10 +794,11 @@ int rb200_carriers_step(rb200_carrier* const* carriers, size_t count, const rb20
                         rb200_step_report* reports, int* statuses) {
     if (!carriers || !params || !reports || !statuses) return RB200_INVALID_ARGUMENT;
     int first_error = RB200_OK;
-    size_t cooperative = 0;
-    for (size_t i = 0; i < count; ++i) cooperative += carriers[i] && carriers[i]->solver.persistent_blocks() > 0;
+    int cooperative[64] = {};  // steps with a cooperative kernel, by device
+    for (size_t i = 0; i < count; ++i)
+        if (carriers[i] && carriers[i]->solver.persistent_blocks() > 0) ++cooperative[carriers[i]->device & 63];
     for (size_t i = 0; i < count; ++i) {
-        statuses[i] = launch_step(carriers[i], &params[i], 0, cooperative > 1);
+        statuses[i] = launch_step(carriers[i], &params[i], 0, carriers[i] && cooperative[carriers[i]->device & 63] > 1);
         if (statuses[i] && !first_error) first_error = statuses[i];
     }
     for (size_t i = 0; i < count; ++i) {
