@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(DCT_THREADS, 2) k_b_dct(const BatchDctJob* __r
     if (st->flags & F_DONE) return;
     block_copy(J, job.J);
     __syncthreads();
-    const float scale = ROW ? (OP == DCT_FORWARD ? st->down : st->up) : 1.0f;
+    const float scale = ROW ? (OP == DCT_FORWARD ? extra_of(st).down : extra_of(st).up) : 1.0f;
     dct_tile_any<ROW, OP>(J, sp.block, J.src64 != nullptr && st->it == 0, scale, reinterpret_cast<float*>(dct_smem));
 }
 
@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(BT) k_b_true_residual(const BatchInstDev* __re
     if (publish_and_check_last<3, 1>(I.part, sp.block, sp.blocks, sums, mx)) {
         fold_partials<3, 1>(I.part, sp.blocks, red, sums, mx);
         if (threadIdx.x == 0) {
-            st->load_mean = dd_value(sums[2]) / g.cells;
+            extra_of(st).load_mean = dd_value(sums[2]) / g.cells;
             decide_true(st, nullptr, dd_value(sums[0]), dd_value(sums[1]), mx[0], flags, g.volume);
         }
     }
@@ -1281,7 +1281,7 @@ int rb200_batch_create(const rb200_grid* grids, size_t count, const rb200_batch_
         const GridDev& g = B->grids[i];
         for (int a = 0; a < 3; ++a) total += 3 * aligned(size_t(g.flen[a]) * sizeof(float));
         total += (B->direct[i] ? 3 : 6) * aligned(size_t(g.cells) * sizeof(double));
-        total += aligned(sizeof(SolveState)) + aligned(sizeof(unsigned));
+        total += aligned(sizeof(SolveStates)) + aligned(sizeof(unsigned));
         total += aligned(size_t(B->part_blocks[i]) * kSlotDoubles * sizeof(double));
         if (B->direct[i]) {
             total += 2 * aligned(size_t(g.cells) * sizeof(float));
@@ -1329,7 +1329,7 @@ int rb200_batch_create(const rb200_grid* grids, size_t count, const rb200_batch_
         double** vec[6] = {&I.b, &I.p, &I.d0, &I.r, &I.r1, &I.d1};
         for (int q = 0; q < (B->direct[i] ? 3 : 6); ++q)
             *vec[q] = reinterpret_cast<double*>(take(size_t(g.cells) * 8));
-        I.st = reinterpret_cast<SolveState*>(take(sizeof(SolveState)));
+        I.st = reinterpret_cast<SolveState*>(take(sizeof(SolveStates)));
         I.part.ticket = reinterpret_cast<unsigned*>(take(sizeof(unsigned)));
         I.part.data = reinterpret_cast<double*>(take(size_t(B->part_blocks[i]) * kSlotDoubles * 8));
         I.step = B->step_d + i;

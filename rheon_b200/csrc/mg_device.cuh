@@ -1136,7 +1136,7 @@ __device__ __forceinline__ void update_first_body(const GridDev& g, const MgLeve
     __shared__ BlockReduce<2, 0> red;
     const int flags = st->flags;
     if (flags & F_STOP) return;
-    const double alpha = st->alpha, mean = st->mean;
+    const double alpha = st->alpha, mean = extra_of(st).mean;
     const double* __restrict__ d = st->dsel ? d1 : d0;
     // r_old is kept: the new residual goes to the other buffer
     const int rsel = st->rsel;
@@ -1207,7 +1207,7 @@ __device__ __forceinline__ void update_first_body(const GridDev& g, const MgLeve
         if (threadIdx.x == 0) {
             st->rsel = rsel ^ 1;
             if (flags & F_PROFILE) return;
-            st->mean = dd_value(sums[1]) / g.cells;
+            extra_of(st).mean = dd_value(sums[1]) / g.cells;
             const int it = st->it + 1;
             st->it = it;
             const double recursive_l2 = sqrt(dd_value(sums[0]));

@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(TILE_THREADS) k_true_residual(GridDev g, Solve
     if (publish_and_check_last<3, 1>(part, block_id3(), nb, sums, mx)) {
         fold_partials<3, 1>(part, nb, red, sums, mx);
         if (tid3() == 0) {
-            st->load_mean = dd_value(sums[2]) / g.cells;
+            extra_of(st).load_mean = dd_value(sums[2]) / g.cells;
             decide_true(st, trace, dd_value(sums[0]), dd_value(sums[1]), mx[0], flags, g.volume);
         }
     }
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(EW) k_mg_update(GridDev g, SolveState* st, dou
     __shared__ BlockReduce<2, 0> red;
     const int flags = st->flags;
     if (flags & F_STOP) return;
-    const double alpha = st->alpha, mean = st->mean;
+    const double alpha = st->alpha, mean = extra_of(st).mean;
     const double* __restrict__ d = st->dsel ? d1 : d0;
     Neu acc;
     double total = 0.0;
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(EW) k_mg_update(GridDev g, SolveState* st, dou
         fold_partials<2, 0>(part, gridDim.x, red, sums, none);
         if (threadIdx.x == 0) {
             if (flags & F_PROFILE) return;
-            st->mean = dd_value(sums[1]) / g.cells;
+            extra_of(st).mean = dd_value(sums[1]) / g.cells;
             int it = st->it + 1;
             st->it = it;
             double recursive_l2 = sqrt(dd_value(sums[0]));
@@ -1337,7 +1337,8 @@ int PcgSolver::init(const GridDev& g, int method, cudaStream_t stream) {
     if ((rc = alloc(&part_.data, size_t(part_blocks_) * 12))) return rc;
     RB200_CUDA(cudaMalloc(&part_.ticket, sizeof(unsigned)));
     RB200_CUDA(cudaMemsetAsync(part_.ticket, 0, sizeof(unsigned), stream_));
-    RB200_CUDA(cudaMalloc(&st_, sizeof(SolveState)));
+    RB200_CUDA(cudaMalloc(reinterpret_cast<void**>(&st_), sizeof(SolveStates)));
+    RB200_CUDA(cudaMemsetAsync(st_, 0, sizeof(SolveStates), stream_));
     RB200_CUDA(cudaMallocHost(&h_st_, 2 * sizeof(SolveState)));
     for (auto& e : ev_) RB200_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     maps_ = make_maps(g, z_, d_[0], d_[1], p_, r_);
@@ -1853,7 +1854,7 @@ constexpr size_t kStaticPartialDoubles = size_t(kStaticMaxBlocks) * kStaticSlotD
 constexpr size_t kStaticDoubles = 4 * size_t(kStaticMaxCells) + kStaticPartialDoubles + kStaticStateDoubles;
 static __device__ __align__(256) double g_static_scratch[kStaticDoubles];
 
-static_assert(sizeof(SolveState) + sizeof(unsigned) <= kStaticStateDoubles * sizeof(double),
+static_assert(sizeof(SolveStates) + sizeof(unsigned) <= kStaticStateDoubles * sizeof(double),
               "state does not fit the static scratch");
 
 // Device address of g_static_scratch per device, resolved once per device
@@ -1913,7 +1914,7 @@ int static_solve_jacobi(const GridDev& g, const double* rhs, double* pressure, d
     B.part.data = B.z + kStaticMaxCells;
     double* state_slot = B.part.data + kStaticPartialDoubles;
     B.st = reinterpret_cast<SolveState*>(state_slot);
-    B.part.ticket = reinterpret_cast<unsigned*>(reinterpret_cast<char*>(state_slot) + sizeof(SolveState));
+    B.part.ticket = reinterpret_cast<unsigned*>(reinterpret_cast<char*>(state_slot) + sizeof(SolveStates));
     B.trace = nullptr;
     B.maps = make_maps(g, B.z, B.d0, B.d1, B.p, B.r);
 

@@ -32,11 +32,25 @@ struct SolveState {
     int flexible;       // beta = z.(r - r_old) / rz_old (flexible CG) instead of rz'/rz
     int trips;          // loop-body passes of the graph-embedded solve
     int rsel;           // flexible method: which residual buffer holds r (the update writes the other)
+};
+
+// What the mixed method keeps beside the state, behind it in one allocation: the
+// cooperative kernels hold the state proper in shared memory for a whole launch
+// (24 bytes more of it cost 0.5 % of a 128^3 step).
+struct SolveExtra {
     // flexible method: the means that the next load of a residual (from b or the
     // true residual) and the next update take out of it
     double load_mean, mean;
-    float down, up;     // direct method: powers of two around its transforms (down up = 1)
+    float down, up;  // direct method: powers of two around its transforms (down up = 1)
 };
+struct SolveStates {
+    SolveState state;
+    SolveExtra extra;
+};
+__host__ __device__ inline SolveExtra& extra_of(SolveState* st) { return reinterpret_cast<SolveStates*>(st)->extra; }
+__host__ __device__ inline const SolveExtra& extra_of(const SolveState* st) {
+    return reinterpret_cast<const SolveStates*>(st)->extra;
+}
 
 enum : int {
     F_STOP = 1,          // iteration kernels are no-ops

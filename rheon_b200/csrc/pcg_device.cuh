@@ -24,8 +24,8 @@ __device__ __forceinline__ void set_transform_scale(SolveState* st, double large
         frexp(largest, &e);
         e = min(126, max(-126, e));
     }
-    st->down = ldexpf(1.0f, -e);
-    st->up = ldexpf(1.0f, e);
+    extra_of(st).down = ldexpf(1.0f, -e);
+    extra_of(st).up = ldexpf(1.0f, e);
 }
 
 // The decision of the start (src/pressure.rs:603-650) from the sums of b, |b|
@@ -60,7 +60,7 @@ __device__ __forceinline__ void decide_init(const GridDev& g, SolveState* st, co
         }
     }
     set_transform_scale(st, m[0]);
-    st->load_mean = sum / g.cells;
+    extra_of(st).load_mean = sum / g.cells;
     double rhs_l2 = sqrt(sq);
     double threshold = fmax(st->absolute, st->relative * rhs_l2);
     if (!isfinite(rhs_l2) || !isfinite(threshold)) {
@@ -145,11 +145,11 @@ __device__ __forceinline__ void load_residual_body(const GridDev& g, SolveState*
     // is in the first (the buffer the V-cycle's first half-sweep reads)
     if (KIND == KIND_MG && sp.block == 0 && threadIdx.x == 0) {
         st->rsel = 0;
-        st->mean = 0.0;
+        extra_of(st).mean = 0.0;
     }
     // ... and keeps the gauge row's residual (mg.hpp); the others eliminate it
     const bool full = KIND == KIND_MG && st->flexible;
-    const double mean = full ? st->load_mean : 0.0;
+    const double mean = full ? extra_of(st).load_mean : 0.0;
     Neu acc;
     for (int c = sp.block * blockDim.x + threadIdx.x; c < g.cells; c += sp.blocks * blockDim.x) {
         double rc = full ? src[c] - mean : (c == 0 ? 0.0 : src[c]);
