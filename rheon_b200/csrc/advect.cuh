@@ -200,8 +200,8 @@ __device__ __forceinline__ void face_velocity(const GridDev& g, const Faces<T>& 
 // multiply-adds; the stored value is clamped to its corners' range, as the
 // reference's sample is. Bound by L1 gathers (40 per face) and issue, about
 // 350 instructions a face where the FP64-style arithmetic in float spent 1270: at
-// 256^3 1780 us before, 790 now for the velocity (issue slots 73 % busy), 748
-// and 320 for the tracer.
+// 256^3 1780 us before, 777 now for the velocity (issue slots 73 % busy), 748
+// and 300 for the tracer.
 struct LatticeF {
     float top, last;  // dims - 1, max(dims - 2, 0)
 };

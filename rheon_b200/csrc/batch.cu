@@ -27,7 +27,7 @@ namespace rb200 {
 namespace {
 
 constexpr int BT = 256;       // threads of the packed elementwise kernels
-constexpr int kItems = 16;    // advected faces per thread
+constexpr int kItems = 16;    // faces per thread of the advection's launch (a thread takes three, a cell's lower faces, a trip)
 constexpr int kCellItems = 64;  // cells per thread of the cell passes (most reduce: a block's reduction covers 16384 cells)
 constexpr int kRowsPerWarp = 16;  // rows per warp of the FCG update and finish (their reductions cover 128 rows)
 constexpr int kPass1Kc = 16;   // z-march length of the direction pass
@@ -57,11 +57,12 @@ __device__ __forceinline__ int batch_entry(const BatchSpans& s, Span& sp) {
 
 // Which instances the direct preconditioner solves: all that it covers, except
 // a band of sizes. It is the faster method at every size measured (us per
-// batched step, direct / multigrid: 32 boxes of 32^3 595 / 2329, 8 of 64x48x32
-// 601 / 2255, 64 boxes of 32^3 to 128^3 9513 / 24191). Boxes of the band keep
-// the V-cycle because the profiled step's report is a published result: a
-// batch with a 64x48x32 box (98304 cells) reports the V-cycle's kernels
-// (tests/test_gpu_batch.py).
+// batched step, direct / multigrid: 32 boxes of 32^3 411 / 2121, 8 of 48^3
+// 462 / 2583, 8 of 64x48x32 421 / 2102). The band follows no measurement: its
+// boxes keep the V-cycle, the method that they had first, because the profiled
+// step's report is a published result, and a batch with a 64x48x32 box (98304
+// cells) reports the V-cycle's kernels (tests/test_gpu_batch.py). Without that
+// promise the rule is direct_supported alone.
 constexpr int kBatchVcycleAbove = 65536, kBatchVcycleUpTo = 98304;
 inline bool batch_direct(const GridDev& g) {
     return direct_supported(g) && !(g.cells > kBatchVcycleAbove && g.cells <= kBatchVcycleUpTo);

@@ -53,16 +53,19 @@ bool direct_supported(const GridDev& g) {
         wmax = std::max(wmax, g.weight[d]);
     }
     // Where it applies it is the faster of the two (us per carrier step, direct /
-    // multigrid: 32^3 200 / 544, 64^3 275 / 768, 128^3 669 / 1764, 512x64x64
-    // 781 / 3226, 256^3 4617 / 8753). Larger axes do not fit the transform's
+    // multigrid: 32^3 177 / 521, 64^3 227 / 734, 128^3 495 / 1752, 512x64x64
+    // 584 / 3060, 256^3 2894 / 7198). Larger axes do not fit the transform's
     // tile. The FP32 rounding of z comes back through K as noise spread over
     // the whole spectrum, which the next iteration reduces by 10^5 or more, so
     // uneven spacings cost an iteration where point relaxation stalls
     // (iterations to 1e-8, direct / multigrid: 96x16x16 with h = (1, 0.02,
     // 0.02), condition 2 10^7, 3 / 262; 64^3 with h = (1, 0.01, 1), condition
-    // 2 10^7, 3 / more than 300). Beyond 10^9 the FP64 residual's own rounding
-    // floor nears 1e-8. Weights near the ends of the FP32 range stay with the
-    // multigrid method too.
+    // 2 10^7, 3 / more than 300). Up to 10^9 it also holds where the FP64
+    // residual's own rounding is the limit, of either method: that floor grows
+    // with the condition and is highest for smooth right-hand sides, which end at
+    // 1e-8 from a condition of 3 10^8 on and at 2 to 4e-8 near 10^9, where noise
+    // still takes 4 iterations to 1e-8. Weights near the ends of the FP32 range
+    // stay with the multigrid method too.
     return longest > 8 && longest <= kDctMaxAxis && top <= 1e9 * low && wmax > 1e-12 && wmax < 1e12;
 }
 

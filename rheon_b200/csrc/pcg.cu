@@ -379,7 +379,11 @@ __global__ void __launch_bounds__(EW) k_mg_update(GridDev g, SolveState* st, dou
 // that holds the sweep's number, which makes a word its own flag. The words lie
 // in the direction buffer that the iteration does not hold (the next pass
 // overwrites it whole); the tags are the bits of signalling NaNs, which no
-// arithmetic leaves there, and both buffers start as zeros.
+// arithmetic leaves there, and both buffers start as zeros. A number returns
+// after 131072 applications, and the words of a solve's last one may lie there
+// that long: they are the reverse sweep's (each of its words takes the place of
+// the forward sweep's word of that face cell), and a reverse sweep's reads come
+// after its own unit's forward sweep, which has written those words again.
 //
 // A block takes the next slot of a queue (slots 0..U-1: the units in wave order
 // jb + kb ascending; U..2U-1: the same list backwards for the reverse sweep). A
@@ -500,7 +504,11 @@ static_assert(sgs_face_slots_fit(), "a face has at most 16 lanes, its slots lie 
 // The incoming faces' warp of a unit: lane q fetches line q of the y face, lane
 // 16 + q of the z face, one step of the unit at a time. The words come through
 // asynchronous copies, since a load into registers would be waited for at the
-// next branch; a copy that came before its word is polled for, and those behind
+// next branch (with strong loads into registers, 63x48x37 takes 29.2 ms a solve
+// for 17.4). Such a copy is a weak access that nothing orders after the other
+// block's relaxed store. It needs no order: it goes to L2, where that store is
+// performed, it returns an old or a new word, each word tells by itself which,
+// and an old one is polled for with strong loads, after which the copies behind
 // it are made again.
 template <bool REV>
 __device__ __forceinline__ void sgs_faces(const GridDev& g, const SgsFlow& f, const SgsUnit& U, int steps,

@@ -83,7 +83,7 @@ struct GridBarrier {
 };
 
 // Work queue of the lexicographic SGS preconditioner (one launch per
-// application, forward and reverse sweep): the units of 16 x 16 lines along x
+// application, forward and reverse sweep): the units of 16 x 8 lines along x
 // in wave order and one state word per unit. The queue and the states are
 // zeroed by the r.z kernel that follows every application, which also counts
 // the applications.

@@ -28,8 +28,9 @@
 //
 // Bound by FP64 issue at 16 warps per SM (70 operations per cell and iteration
 // without contraction: 9.2 us at 128^3 on the 128 SMs its bricks occupy, 22.6 us
-// measured) and, on small grids, by the two reductions (about 2.3 us each:
-// butterflies of dependent FP64 additions, 0.5 us one way between SMs).
+// measured) and, on small grids, by the two reductions (about 2.3 us each of the
+// 5.4 at 32^3: butterflies of dependent FP64 additions in the block and in the
+// fold, 0.5 us one way between SMs).
 #include <algorithm>
 #include <type_traits>
 
