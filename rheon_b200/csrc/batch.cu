@@ -284,10 +284,11 @@ __global__ void __launch_bounds__(DCT_THREADS, 2) k_b_dct(const BatchDctJob* __r
     Span sp;
     const BatchDctJob& job = jobs[batch_entry(spans, sp)];
     const SolveState* st = job.st;
-    if (st->flags & F_DONE) return;
+    const int flags = st->flags;
+    if (flags & F_DONE) return;
     block_copy(J, job.J);
     __syncthreads();
-    const float scale = ROW ? (OP == DCT_FORWARD ? extra_of(st).down : extra_of(st).up) : 1.0f;
+    const float scale = ROW ? transform_scale(flags, OP != DCT_FORWARD) : 1.0f;
     dct_tile_any<ROW, OP>(J, sp.block, J.src64 != nullptr && st->it == 0, scale, reinterpret_cast<float*>(dct_smem));
 }
 

@@ -15,9 +15,9 @@ __global__ void __launch_bounds__(DCT_THREADS, 2) k_dct(const __grid_constant__ 
     pdl_wait();
     extern __shared__ float4 dct_smem[];
     const int flags = st->flags;
-    const float scale = ROW ? (OP == DCT_FORWARD ? extra_of(st).down : extra_of(st).up) : 1.0f;
     if (flags & F_DONE) return;
     const bool cold = J.src64 != nullptr && st->it == 0 && !(flags & F_WARM);
+    const float scale = ROW ? transform_scale(flags, OP != DCT_FORWARD) : 1.0f;
     dct_tile_any<ROW, OP>(J, blockIdx.x, cold, scale, reinterpret_cast<float*>(dct_smem));
 }
 

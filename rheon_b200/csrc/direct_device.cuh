@@ -505,19 +505,20 @@ __device__ __forceinline__ void decide_refined(SolveState* st, rb200_trace* trac
     const double div = maximum * st->dt / volume;
     const double l2 = sqrt(squared);
     st->recursive_l2 = l2;
-    set_transform_scale(st, maximum);
     if (trace && it >= 1) {
         rb200_trace& t = trace[it - 1];
         t.alpha = 1.0;  // p += z
         t.recursive_l2 = l2;
         t.checked = 1;
     }
-    flags &= ~(F_STOP | F_NEED_TRUE);
+    flags = with_transform_scale(flags & ~(F_STOP | F_NEED_TRUE), maximum);
     if (!isfinite(squared) || !isfinite(div)) {
         breakdown(st, it, flags);
         return;
     }
-    const double before = st->true_max;
+    // what FP32 holds of a residual below its normal range has nothing more to
+    // give than an iteration that did not halve it
+    const bool spent = !seed && maximum < 0x1p-126 && !(maximum < 0.5 * st->true_max);
     st->true_l2 = l2;
     st->true_max = maximum;
     st->true_div = div;
@@ -525,8 +526,8 @@ __device__ __forceinline__ void decide_refined(SolveState* st, rb200_trace* trac
         finish(st, RB200_OK, flags);
     else if (it == st->max_it)
         finish(st, RB200_ITERATION_LIMIT, flags);
-    else if (!seed && maximum < 0x1p-126 && !(maximum < 0.5 * before))
-        breakdown(st, it, flags);  // what FP32 holds of the residual below its normal range has nothing more to give
+    else if (spent)
+        breakdown(st, it, flags);
     else
         st->flags = flags;
 }

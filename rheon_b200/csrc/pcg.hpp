@@ -34,14 +34,13 @@ struct SolveState {
     int rsel;           // flexible method: which residual buffer holds r (the update writes the other)
 };
 
-// What the mixed method keeps beside the state, behind it in one allocation: the
-// cooperative kernels hold the state proper in shared memory for a whole launch
-// (24 bytes more of it cost 0.5 % of a 128^3 step).
+// What the flexible method keeps beside the state, behind it in one allocation:
+// the cooperative kernels hold the state proper in shared memory for a whole
+// launch (24 bytes more of it cost 0.5 % of a 128^3 step).
 struct SolveExtra {
-    // flexible method: the means that the next load of a residual (from b or the
+    // the means that the next load of a residual (from b or the
     // true residual) and the next update take out of it
     double load_mean, mean;
-    float down, up;  // direct method: powers of two around its transforms (down up = 1)
 };
 struct SolveStates {
     SolveState state;
@@ -59,8 +58,10 @@ enum : int {
     F_DONE = 8,          // solve finished; status is final
     F_NEED_REPLACE = 16, // replace r by the true residual, re-precondition
     F_PROFILE = 64,      // timing mode: passes do their work, decisions are skipped
-    F_WARM = 128         // seeded solve: p holds the caller's initial pressure
+    F_WARM = 128,        // seeded solve: p holds the caller's initial pressure
+    F_SCALE = 0xff0000   // direct method: the exponent of its transforms' scale, signed
 };
+constexpr int F_SCALE_SHIFT = 16;
 constexpr int ST_RUNNING = -1;
 
 // Tensor maps of the solver's vectors for the TMA slab loads (unused when the

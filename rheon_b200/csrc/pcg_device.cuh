@@ -17,15 +17,21 @@ constexpr double kEps = 2.220446049250313e-16;
 // that they read and the correction that they write, from the residual's largest
 // value. Inside, sums are up to sqrt(N) larger than the residual and products
 // 1e-7 smaller, so a residual that FP32 just holds would leave its range on
-// either side. Scaling by a power of two changes no other bit.
-__device__ __forceinline__ void set_transform_scale(SolveState* st, double largest) {
+// either side. Scaling by a power of two changes no other bit. The exponent lies
+// in the flags, which every kernel reads at its start: as a value of its own, a
+// second load before the transforms' first, it cost a 64^3 step 1 us.
+__device__ __forceinline__ int with_transform_scale(int flags, double largest) {
     int e = 0;
     if (largest > 0.0 && !(largest >= 0x1p-64 && largest <= 0x1p64)) {
         frexp(largest, &e);
         e = min(126, max(-126, e));
     }
-    extra_of(st).down = ldexpf(1.0f, -e);
-    extra_of(st).up = ldexpf(1.0f, e);
+    return (flags & ~F_SCALE) | (e & 0xff) << F_SCALE_SHIFT;
+}
+// 2^-e in front of the transforms (`up` false), 2^e behind them.
+__device__ __forceinline__ float transform_scale(int flags, bool up) {
+    const int e = int(unsigned(flags) << (24 - F_SCALE_SHIFT)) >> 24;
+    return __int_as_float((127 + (up ? e : -e)) << 23);
 }
 
 // The decision of the start (src/pressure.rs:603-650) from the sums of b, |b|
@@ -59,7 +65,7 @@ __device__ __forceinline__ void decide_init(const GridDev& g, SolveState* st, co
             return;
         }
     }
-    set_transform_scale(st, m[0]);
+    flags = with_transform_scale(flags, m[0]);
     extra_of(st).load_mean = sum / g.cells;
     double rhs_l2 = sqrt(sq);
     double threshold = fmax(st->absolute, st->relative * rhs_l2);
@@ -90,6 +96,7 @@ __device__ __forceinline__ void decide_init(const GridDev& g, SolveState* st, co
         finish(st, RB200_ITERATION_LIMIT, flags);
         return;
     }
+    st->flags = flags;
 }
 
 // ------------------------------------------------------------------ init
